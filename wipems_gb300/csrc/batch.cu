@@ -43,7 +43,7 @@ __global__ void k_batch_advance(const AdvJob* __restrict__ jobs, double eps0, do
     const AdvJob& J = jobs[blockIdx.x];
     const int ts = *J.d_ts + 1;
     const int sample = (J.interval > 0 && (ts % J.interval) == 0) ? 1 : 0;
-    advance_sample(J.d_ts, 1, sample, J.ps, J.g, J.energy_valid, eps0, mue0, threadIdx.x, blockDim.x);
+    advance_sample(J.d_ts, 1, sample, J.ps, J.g, J.energy_valid, eps0, mue0);
     __syncthreads();
     if (threadIdx.x < 4) J.out[threadIdx.x] = J.ctl[threadIdx.x];
 }

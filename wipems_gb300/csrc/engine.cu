@@ -159,13 +159,20 @@ int launch_step(fdtd_engine_s* e, int ts_off, bool energy) {
     return check_launch();
 }
 
+// n timesteps from the fields of numTS (the counter itself is advanced
+// after them); energy: the last one writes the energy segments
+int launch_steps(fdtd_engine_s* e, uint32_t n, bool energy) {
+    int rc = FDTD_OK;
+    for (uint32_t k = 0; k < n && rc == FDTD_OK; ++k) rc = launch_step(e, (int)k, energy && k + 1 == n);
+    return rc;
+}
+
 int launch_advance(fdtd_engine_s* e, int adv, bool sample, bool energy_valid) {
-    if (sample && energy_valid && adv > 0) {  // the last current kernel wrote the energy segments
-        k_energy_planes<<<e->N[0] - 1, 256, 0, e->stream>>>(e->g);
-        e->last_launches += 1;
-    }
-    k_advance_sample<<<1, 256, 0, e->stream>>>(e->p_ts(), adv, sample ? 1 : 0, e->ps, e->g, energy_valid ? 1 : 0,
-                                                kEps0, kMue0);
+    // after timesteps the last current update left energy segments to sum
+    const bool planes = sample && energy_valid && adv > 0;
+    k_advance_sample<<<planes ? e->N[0] - 1 : 1, 256, 0, e->stream>>>(e->p_ts(), adv, sample ? 1 : 0, e->ps, e->g,
+                                                                       energy_valid ? 1 : 0, planes ? 1 : 0,
+                                                                       e->ticket.p, kEps0, kMue0);
     e->last_launches += 1;
     return check_launch();
 }
@@ -238,11 +245,11 @@ int build_chunk_graph(fdtd_engine_s* e) {
     if (e->chunk) return FDTD_OK;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = FDTD_OK;
+    int rc;
     const uint64_t saved = e->last_launches;
-    for (uint32_t k = 0; k < e->interval && rc == FDTD_OK; ++k)
-        rc = launch_step(e, (int)k, e->energy_on_probe && (k + 1 == e->interval));
+    rc = launch_steps(e, e->interval, e->energy_on_probe);
     if (rc == FDTD_OK) rc = launch_advance(e, (int)e->interval, true, e->energy_on_probe);
+    e->chunk_launches = e->last_launches - saved;
     e->last_launches = saved;
     cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
     if (rc != FDTD_OK) {
@@ -452,6 +459,7 @@ int reset_state(fdtd_engine_s* e) {
     for (DevBuf<float>* b : {&e->AVx, &e->LVx, &e->AIx, &e->LIx})
         if (b->p) CK(cudaMemsetAsync(b->p, 0, b->n * sizeof(float), s));
     CK(cudaMemsetAsync(e->ctl.p, 0, 4 * sizeof(int), s));
+    CK(cudaMemsetAsync(e->ticket.p, 0, sizeof(unsigned), s));
     if (e->d_fd.p) CK(cudaMemsetAsync(e->d_fd.p, 0, e->d_fd.n * sizeof(double), s));
     if (e->mur_buf.p) CK(cudaMemsetAsync(e->mur_buf.p, 0, e->mur_buf.n * sizeof(float), s));
     if (e->rlc_state.p) CK(cudaMemsetAsync(e->rlc_state.p, 0, e->rlc_state.n * sizeof(float), s));
@@ -599,7 +607,7 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
         (rc = e->sigC.alloc(std::max<uint32_t>(1, c->sig_len), tot, e->stream)))
         return rc;
     if ((rc = e->ctl.alloc(4, tot, e->stream)) || (rc = e->d_eacc.alloc(4, tot, e->stream)) ||
-        (rc = e->d_energy_tmp.alloc(2, tot, e->stream)))
+        (rc = e->d_energy_tmp.alloc(2, tot, e->stream)) || (rc = e->ticket.alloc(1, tot, e->stream)))
         return rc;
     // energy segments: one float pair per (x < Nx-1, y < Ny-1, 32-node z tile)
     const int nzt = ((int)e->N[2] - 1 + 31) / 32;
@@ -1006,24 +1014,22 @@ int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
     const bool fd_on = e->fd_interval && !e->h_freq.empty() && e->ps.nprobe;
     uint32_t left = n;
     while (left > 0) {
-        // steps to the next frequency-domain step (a chunk graph may end on
-        // it, not pass it)
-        const uint32_t to_fd = fd_on ? e->fd_interval - (e->ts % e->fd_interval) : ~0u;
-        if (e->interval && e->use_graphs && e->chunk && (e->ts % e->interval) == 0 && left >= e->interval &&
-            to_fd >= e->interval) {
+        // run to the next sample or frequency-domain step; the counter
+        // advances once per run
+        uint32_t run = std::min(left, 1u << 16);
+        if (e->interval) run = std::min(run, e->interval - e->ts % e->interval);
+        if (fd_on) run = std::min(run, e->fd_interval - e->ts % e->fd_interval);
+        if (e->chunk && run == e->interval) {
             CK(cudaGraphLaunch(e->chunk, e->stream));
-            e->last_launches += (e->fused ? 1 : 2) * (uint64_t)e->interval + 1 + (e->energy_on_probe ? 1 : 0);
-            e->ts += e->interval;
-            left -= e->interval;
-            if (to_fd == e->interval && (rc = launch_fd(e, e->ts))) return rc;
-            continue;
+            e->last_launches += e->chunk_launches;
+        } else {
+            const bool sample = e->interval && (e->ts + run) % e->interval == 0;
+            if ((rc = launch_steps(e, run, sample && e->energy_on_probe))) return rc;
+            if ((rc = launch_advance(e, (int)run, sample, e->energy_on_probe))) return rc;
         }
-        const bool sample = e->interval && ((e->ts + 1) % e->interval) == 0;
-        if ((rc = launch_step(e, 0, sample && e->energy_on_probe))) return rc;
-        if ((rc = launch_advance(e, 1, sample, e->energy_on_probe))) return rc;
-        e->ts += 1;
-        left -= 1;
-        if (fd_on && (e->ts % e->fd_interval) == 0 && (rc = launch_fd(e, e->ts))) return rc;
+        e->ts += run;
+        left -= run;
+        if (fd_on && e->ts % e->fd_interval == 0 && (rc = launch_fd(e, e->ts))) return rc;
     }
     CK(cudaEventRecord(e->ev1, e->stream));
     e->pending = true;
@@ -1357,7 +1363,7 @@ int fdtd_engine_energy(fdtd_engine_t e, double* energy) {
     const dim3 grid((unsigned)g.nzt, (e->N[1] - 1 + 7) / 8, e->N[0] - 1);
     k_energy_segments<<<grid, dim3(32, 8), 0, e->stream>>>(g);
     k_energy_planes<<<e->N[0] - 1, 256, 0, e->stream>>>(g);
-    k_energy_total<<<1, 32, 0, e->stream>>>(g, kEps0, kMue0, e->d_energy_tmp.p);
+    k_energy_total<<<1, 256, 0, e->stream>>>(g, kEps0, kMue0, e->d_energy_tmp.p);
     CK(cudaGetLastError());
     double h = 0;
     CK(cudaMemcpyAsync(&h, e->d_energy_tmp.p, sizeof(h), cudaMemcpyDeviceToHost, e->stream));

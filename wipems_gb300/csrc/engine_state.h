@@ -115,6 +115,7 @@ struct fdtd_engine_s {
     int* p_done() const { return ctl.p + 3; }
     DevBuf<double> d_eacc;  // [2]: running energy maximum (end criterion)
     DevBuf<double> d_energy_tmp;
+    DevBuf<unsigned> ticket;  // blocks of a sampling launch that have finished (k_advance_sample)
     DevBuf<ProbeEntry> now_entries;  // fdtd_engine_probe_now scratch, grown on demand
     DevBuf<double> now_misc;
     DevBuf<float2> eseg;    // energy segments (DevGrid::eseg)
@@ -176,6 +177,7 @@ struct fdtd_engine_s {
     uint32_t num_tuples_e = 0, num_tuples_h = 0, upml_nodes = 0, ade_nodes = 0;
     uint64_t device_bytes = 0;
     cudaGraphExec_t chunk = nullptr;
+    uint64_t chunk_launches = 0;  // kernels in it
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0;
     uint64_t last_launches = 0;

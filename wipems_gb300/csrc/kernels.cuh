@@ -293,6 +293,58 @@ static __global__ void k_fd_accumulate(const int* d_ts, int expect_ts, ProbeSet 
     if (tid == 0) *fd.count += 1;
 }
 
+// Sum of a pair over a 256-thread block in a fixed order: a shuffle tree in
+// each warp, then the warps in order.  Thread 0 returns the sums.
+__device__ __forceinline__ double2 block_sum(double a, double b) {
+    __shared__ double sa[8], sb[8];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, off);
+        b += __shfl_down_sync(0xffffffffu, b, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sa[threadIdx.x >> 5] = a;
+        sb[threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    double2 r = make_double2(0.0, 0.0);
+    if (threadIdx.x == 0) {
+        for (int w = 0; w < 8; ++w) {
+            r.x += sa[w];
+            r.y += sb[w];
+        }
+    }
+    return r;
+}
+
+// Sum of the energy segments of plane x (256 threads: each sums a strided
+// share in double, then block_sum); thread 0 returns the pair.
+__device__ __forceinline__ double2 plane_energy(const DevGrid& g, int x) {
+    const long long n = (long long)(g.Ny - 1) * g.nzt;
+    const float2* seg = g.eseg + (long long)x * n;
+    double a = 0.0, b = 0.0;
+    for (long long i = threadIdx.x; i < n; i += 256) {
+        const float2 v = seg[i];
+        a += (double)v.x;
+        b += (double)v.y;
+    }
+    return block_sum(a, b);
+}
+
+// Sum of the plane sums, in an order fixed by the grid: each of 256 threads
+// takes every 256th plane, then block_sum.  (One thread walking the planes is
+// a chain of dependent double additions: a sample on 65 planes took 12.4 us.)
+// The plane sums may come from other blocks of the same launch: read in L2.
+__device__ __forceinline__ double2 total_energy(const DevGrid& g) {
+    double a = 0.0, b = 0.0;
+    for (int x = threadIdx.x; x < g.Nx - 1; x += 256) {
+        const double2 p = __ldcg(&g.eplane[x]);
+        a += p.x;
+        b += p.y;
+    }
+    return block_sum(a, b);
+}
+
 // Advances numTS by adv (Engine::IterateTS ++numTS) and, when sample is set,
 // records one probe/energy sample row (ProcessIntegral::Process): the probe
 // sums (ProcessVoltage / ProcessCurrent) as warp reductions in double.
@@ -300,11 +352,11 @@ static __global__ void k_fd_accumulate(const int* d_ts, int expect_ts, ProbeSet 
 // openEMS::RunFDTD's loop ends (openems.cpp:1285-1314): at the first sample
 // whose energy is <= end_crit times the largest energy seen so far, or at
 // stop_ts timesteps; a stopped job's kernels and samplers do nothing.
-// tid / nthr: the calling thread's linear index in the block and the
-// block's thread count (a multiple of 32); every thread of the block calls.
+// Every thread of a 256-thread block calls.
 __device__ __forceinline__ void advance_sample(int* d_ts, int adv, int sample, const ProbeSet& ps, const DevGrid& g,
-                                               int energy_valid, double eps0, double mue0, int tid, int nthr) {
+                                               int energy_valid, double eps0, double mue0) {
     __shared__ int s_ts, s_row, s_done;
+    const int tid = threadIdx.x;
     if (tid == 0) {
         s_row = -1;
         s_done = *ps.d_done;
@@ -330,22 +382,15 @@ __device__ __forceinline__ void advance_sample(int* d_ts, int adv, int sample, c
     if (!sample || s_row < 0) return;
     double* rec = ps.ring + (long long)s_row * ps.row_doubles;
     const int warp = tid >> 5, lane = tid & 31;
-    const int nwarps = nthr >> 5;
-    for (int p = warp; p < ps.nprobe; p += nwarps) {
+    for (int p = warp; p < ps.nprobe; p += 8) {
         const double acc = probe_value(ps, g, p, s_ts, lane);
         if (lane == 0) rec[2 + p] = acc * ps.weight[p];
     }
+    const double2 sum = energy_valid ? total_energy(g) : make_double2(0.0, 0.0);
     if (tid == 0) {
         rec[0] = (double)s_ts;
         if (energy_valid) {
-            // the plane sums in x order (fixed by the grid)
-            double a = 0.0, b = 0.0;
-            for (int x = 0; x < g.Nx - 1; ++x) {
-                const double2 p = g.eplane[x];
-                a += p.x;
-                b += p.y;
-            }
-            double e = eps0 * a + mue0 * b;
+            double e = eps0 * sum.x + mue0 * sum.y;
             if (!isfinite(e)) atomicOr(ps.d_err, 2);
             rec[1] = e;
             if (ps.end_crit > 0.0) {
@@ -357,39 +402,6 @@ __device__ __forceinline__ void advance_sample(int* d_ts, int adv, int sample, c
             rec[1] = -1.0;
         }
     }
-}
-
-// Sum of the energy segments of plane x in a fixed order (256 threads: each
-// sums a strided share in double, then a fixed shuffle / shared-memory
-// tree); thread 0 returns the pair.
-__device__ __forceinline__ double2 plane_energy(const DevGrid& g, int x) {
-    __shared__ double sa[8], sb[8];
-    const long long n = (long long)(g.Ny - 1) * g.nzt;
-    const float2* seg = g.eseg + (long long)x * n;
-    double a = 0.0, b = 0.0;
-    for (long long i = threadIdx.x; i < n; i += 256) {
-        const float2 v = seg[i];
-        a += (double)v.x;
-        b += (double)v.y;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, off);
-        b += __shfl_down_sync(0xffffffffu, b, off);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        sa[threadIdx.x >> 5] = a;
-        sb[threadIdx.x >> 5] = b;
-    }
-    __syncthreads();
-    double2 r = make_double2(0.0, 0.0);
-    if (threadIdx.x == 0) {
-        for (int w = 0; w < 8; ++w) {
-            r.x += sa[w];
-            r.y += sb[w];
-        }
-    }
-    return r;
 }
 
 // one probe integral of the current fields (one warp), written to out[0]
@@ -404,9 +416,32 @@ static __global__ void __launch_bounds__(256) k_energy_planes(const DevGrid g) {
     if (threadIdx.x == 0) g.eplane[blockIdx.x] = r;
 }
 
-static __global__ void k_advance_sample(int* d_ts, int adv, int sample, ProbeSet ps, const DevGrid g, int energy_valid,
-                                        double eps0, double mue0) {
-    advance_sample(d_ts, adv, sample, ps, g, energy_valid, eps0, mue0, threadIdx.x, blockDim.x);
+// True in every thread of the block that arrives last of `blocks` (its
+// reads then see what the others wrote before); the ticket is back at zero
+// for the next launch.
+__device__ __forceinline__ bool last_block(unsigned* ticket, unsigned blocks) {
+    __shared__ int s_last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(ticket, blocks - 1) == blocks - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
+// Counter, probe sample and energy of a chunk of timesteps in one launch:
+// with energy one block per x plane sums its segments and the last one to
+// finish takes the sample; without it one block does.
+static __global__ void __launch_bounds__(256) k_advance_sample(int* d_ts, int adv, int sample, ProbeSet ps,
+                                                               const DevGrid g, int energy_valid, int planes,
+                                                               unsigned* ticket, double eps0, double mue0) {
+    if (planes) {
+        const double2 r = plane_energy(g, blockIdx.x);
+        if (threadIdx.x == 0) g.eplane[blockIdx.x] = r;
+        if (!last_block(ticket, gridDim.x)) return;
+    }
+    advance_sample(d_ts, adv, sample, ps, g, energy_valid, eps0, mue0);
 }
 
 // ------------------------------------------------------------- Mur ABC
@@ -747,16 +782,10 @@ static __global__ void k_energy_segments(const DevGrid g) {
     energy_segment(g, x, y, zt, act, y < g.Ny - 1, v[0], v[1], v[2], c[0], c[1], c[2]);
 }
 
-// eps0 * sum E + mue0 * sum H over the planes in x order (one thread)
-static __global__ void k_energy_total(const DevGrid g, double eps0, double mue0, double* out) {
-    if (threadIdx.x != 0) return;
-    double a = 0.0, b = 0.0;
-    for (int x = 0; x < g.Nx - 1; ++x) {
-        const double2 p = g.eplane[x];
-        a += p.x;
-        b += p.y;
-    }
-    out[0] = eps0 * a + mue0 * b;
+// eps0 * sum E + mue0 * sum H over the planes (one block of 256 threads)
+static __global__ void __launch_bounds__(256) k_energy_total(const DevGrid g, double eps0, double mue0, double* out) {
+    const double2 s = total_energy(g);
+    if (threadIdx.x == 0) out[0] = eps0 * s.x + mue0 * s.y;
 }
 
 }  // namespace wipems
