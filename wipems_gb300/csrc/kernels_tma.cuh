@@ -451,8 +451,12 @@ __device__ __forceinline__ bool curr_tile(const DevGrid& g, const TmaMaps& m, co
     return !aborted;
 }
 
+// The next 128-byte boundary of the dynamic shared memory, by an offset:
+// rounding the pointer as an integer loses its address space, and every read
+// of the ring became a generic load (one in ten instructions of the voltage
+// kernel; 119 x 102 x 151 lines with UPML 39.4 against 38.1 us per step).
 __device__ __forceinline__ float* aligned_smem(float* raw) {
-    return reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(raw) + 127) & ~(uintptr_t)127);
+    return raw + ((0u - smem_u32(raw)) & 127u) / 4u;
 }
 
 __device__ __forceinline__ void init_ring(uint64_t* bars, int STAGES) {
