@@ -181,7 +181,7 @@ int launch_advance(fdtd_engine_s* e, int adv, bool sample, bool energy_valid) {
 int launch_fd(fdtd_engine_s* e, uint32_t ts) {
     if (!e->fd_interval || e->h_freq.empty() || e->ps.nprobe == 0) return FDTD_OK;
     const size_t sm = std::max<size_t>(8, (size_t)e->ps.nprobe * sizeof(double));
-    k_fd_accumulate<<<1, 256, sm, e->stream>>>(e->p_ts(), (int)ts, e->ps, e->g, e->fd);
+    k_fd_accumulate<<<1, 256, sm, e->stream>>>(e->p_ts(), (int)ts, e->ps, e->g, e->fd, (int)ts, 0, 1, 0);
     e->last_launches += 1;
     return check_launch();
 }
@@ -275,7 +275,8 @@ int start(fdtd_engine_s* e) {
     if (!e->started) {
         if ((rc = upload_probes(e))) return rc;
         e->started = true;
-        if (e->interval && e->use_graphs && (rc = build_chunk_graph(e))) return rc;
+        if (e->res_candidate && (rc = setup_resident(e))) return rc;
+        if (e->interval && e->use_graphs && !e->resident && (rc = build_chunk_graph(e))) return rc;
     }
     if (e->need_initial_sample) {
         e->need_initial_sample = false;
@@ -460,6 +461,7 @@ int reset_state(fdtd_engine_s* e) {
         if (b->p) CK(cudaMemsetAsync(b->p, 0, b->n * sizeof(float), s));
     CK(cudaMemsetAsync(e->ctl.p, 0, 4 * sizeof(int), s));
     CK(cudaMemsetAsync(e->ticket.p, 0, sizeof(unsigned), s));
+    if (e->res_ll.p) CK(cudaMemsetAsync(e->res_ll.p, 0, e->res_ll.n * sizeof(ulonglong2), s));
     if (e->d_fd.p) CK(cudaMemsetAsync(e->d_fd.p, 0, e->d_fd.n * sizeof(double), s));
     if (e->mur_buf.p) CK(cudaMemsetAsync(e->mur_buf.p, 0, e->mur_buf.n * sizeof(float), s));
     if (e->rlc_state.p) CK(cudaMemsetAsync(e->rlc_state.p, 0, e->rlc_state.n * sizeof(float), s));
@@ -500,6 +502,16 @@ int upload_half(fdtd_engine_s* e, const HalfTables& T, DevHalfBufs& B, DevHalf& 
     D.adex = reinterpret_cast<const float4*>(B.adex.p);
     D.ntup = (int)T.num_tuples;
     return FDTD_OK;
+}
+
+// Whether runs of timesteps may stay in shared memory (if the grid fits, see
+// setup_resident): the default kernel choice with the default tiling
+// (explicit tilings are the half-step kernels'), 16-bit indices, no
+// Lorentz/Drude nodes, no passes between the half-steps (Mur faces, lumped RLC edges), and no end criterion
+// (which is decided sample by sample).
+bool resident_applies(const fdtd_engine_s* e, const fdtd_cop_s* c, const fdtd_engine_opts* o) {
+    if (o && (o->kernel != 0 || o->tile_y > 0 || o->x_chunk > 0 || o->stages > 0)) return false;
+    return c->E.idx16 && c->H.idx16 && !(e->feat & (FEAT_ADE | FEAT_ADEX)) && c->mur.empty() && !c->rlc.size() && e->end_crit == 0.0;
 }
 
 int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine_s* e) {
@@ -773,6 +785,7 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
                                                          : StageLayout<uint32_t, false, true>::smem(e->stages));
         if (need > 48 * 1024 && (rc = set_smem_attrs((int)need))) return rc;
     }
+    e->res_candidate = resident_applies(e, c, opts);
     return reset_state(e);
 }
 
@@ -1014,6 +1027,13 @@ int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
     const bool fd_on = e->fd_interval && !e->h_freq.empty() && e->ps.nprobe;
     uint32_t left = n;
     while (left > 0) {
+        if (e->resident) {
+            const uint32_t run = resident_run(e, left);
+            if ((rc = launch_resident(e, run))) return rc;
+            e->ts += run;
+            left -= run;
+            continue;
+        }
         // run to the next sample or frequency-domain step; the counter
         // advances once per run
         uint32_t run = std::min(left, 1u << 16);
@@ -1269,6 +1289,8 @@ int fdtd_engine_restore(fdtd_engine_t e, const void* buf, uint64_t size) {
         if (b) CK(cudaMemcpyAsync(q.p, o, b, cudaMemcpyHostToDevice, e->stream));
         o += b;
     }
+    // numTS may go back: no exchange word of a later timestep may stay
+    if (e->res_ll.p) CK(cudaMemsetAsync(e->res_ll.p, 0, e->res_ll.n * sizeof(ulonglong2), e->stream));
     CK(cudaStreamSynchronize(e->stream));
     e->ts = h.ts;
     e->done = h.done != 0;

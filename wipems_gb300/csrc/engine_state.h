@@ -12,6 +12,7 @@
 #include "fdtd_host.h"
 #include "kernels.cuh"
 #include "kernels_fused.cuh"
+#include "kernels_resident.cuh"
 #include "kernels_tma.cuh"
 
 namespace wipems {
@@ -167,6 +168,16 @@ struct fdtd_engine_s {
     bool use_tma = true;
     bool fused = false;      // single-pass kernel, double-buffered fields
     FusedMaps fmaps{};
+    // resident timesteps (kernels_resident.cuh): runs of timesteps with the
+    // fields in shared memory, back in V / I at the end of each run
+    bool res_candidate = false, resident = false;
+    ResArgs ra{};
+    const void* res_kernel = nullptr;
+    int res_smem = 0, res_threads = 0, res_samples = 0;  // samples one run can hold
+    DevBuf<ulonglong2> res_ll;             // exchange pairs
+    DevBuf<float> res_pval, res_fdval;     // probe entry values of a run's samples / frequency-domain steps
+    DevBuf<float2> res_seg;                // their energy segments and plane sums
+    DevBuf<double2> res_plane;
     // field buffers holding the fields at the current numTS
     float* cur_V() const { return (fused && (ts & 1)) ? V2.p : V.p; }
     float* cur_I() const { return (fused && (ts & 1)) ? I2.p : I.p; }
@@ -213,6 +224,13 @@ inline int auto_x_chunk(const std::vector<const uint32_t*>& lines, uint64_t resi
     }
     return best;
 }
+
+// resident.cu
+// boxes per axis, at most `blocks` of at most `nodes`; false if the grid does not fit
+bool resident_plan(const int cov[3], int blocks, int nodes, int p[3]);
+int setup_resident(fdtd_engine_s* e);                    // sets e->resident if the grid fits
+uint32_t resident_run(const fdtd_engine_s* e, uint32_t n);  // timesteps the next launch can take, at most n
+int launch_resident(fdtd_engine_s* e, uint32_t n);       // n timesteps and their samples
 
 // engine.cu helpers used by the batched path
 int engine_start(fdtd_engine_s* e);        // upload probes, graph, ts = 0 sample

@@ -202,6 +202,7 @@ struct ProbeSet {
     int* d_done;                // end criterion met (0 / 1)
     double end_crit;            // > 0: stop once energy <= end_crit * max energy
     int stop_ts;                // > 0 (with end_crit): stop at this numTS
+    const float* vals;          // the entries' values, gathered before (null: read the fields)
 };
 
 // Integral of probe p over the fields of numTS ts, by one warp: the lanes
@@ -223,7 +224,7 @@ __device__ __forceinline__ double probe_sum(const ProbeSet& ps, const DevGrid& g
         if (base + lane < last) {
             const ProbeEntry pe = ps.entries[base + lane];
             const float* f = pe.field ? (odd ? g.I2 : g.I) : (odd ? g.V2 : g.V);
-            v = f[(long long)pe.comp * g.comp + pe.off];
+            v = ps.vals ? ps.vals[base + lane] : f[(long long)pe.comp * g.comp + pe.off];
             sg = pe.sign;
         }
         const int cnt = min(32, last - base);
@@ -245,6 +246,7 @@ __device__ __forceinline__ double probe_value(const ProbeSet& ps, const DevGrid&
     const double dv = ps.div[p];
     if (dv == 0.0) return probe_sum(ps, g, p, ts, lane);
     if (dv < 0.0) return 0.0;
+    if (ps.vals) return (double)ps.vals[ps.first[p]] / dv;
     const ProbeEntry pe = ps.entries[ps.first[p]];
     const bool odd = g.V2 && (ts & 1);
     const float* f = pe.field ? (odd ? g.I2 : g.I) : (odd ? g.V2 : g.V);
@@ -267,30 +269,38 @@ struct FdSet {
 
 // One block; dynamic shared memory: nprobe doubles.  expect_ts: the numTS
 // the host launched this for (a job that stopped on its end criterion
-// earlier has a smaller numTS and is left alone).
-static __global__ void k_fd_accumulate(const int* d_ts, int expect_ts, ProbeSet ps, const DevGrid g, FdSet fd) {
+// earlier has a smaller numTS and is left alone).  One step from the fields,
+// or `count` steps from first_ts on, every `every` timesteps, whose probe
+// entry values a run of timesteps gathered (ps.vals, nentry per step).
+static __global__ void k_fd_accumulate(const int* d_ts, int expect_ts, ProbeSet ps, const DevGrid g, FdSet fd,
+                                       int first_ts, int every, int count, int nentry) {
     extern __shared__ double s_val[];
     __shared__ int s_go;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     if (tid == 0) s_go = (*d_ts == expect_ts);
     __syncthreads();
     if (!s_go) return;
-    for (int p = warp; p < ps.nprobe; p += nwarps) {
-        const double acc = probe_value(ps, g, p, expect_ts, lane);
-        if (lane == 0) s_val[p] = acc * ps.weight[p];
-    }
-    __syncthreads();
     const int n = ps.nprobe * fd.nfreq;
-    for (int k = tid; k < n; k += blockDim.x) {
-        const int p = k / fd.nfreq, f = k - p * fd.nfreq;
-        const double t = ((double)expect_ts + 0.5 * (double)fd.dual[p]) * fd.dT;
-        double sn, cs;
-        sincospi(2.0 * fd.freq[f] * t, &sn, &cs);  // exp(-2 pi i f t) = cs - i sn
-        const double v = s_val[p] * fd.scale;
-        fd.acc[2 * k] += v * cs;
-        fd.acc[2 * k + 1] -= v * sn;
+    for (int m = 0; m < count; ++m) {
+        const int ts = first_ts + m * every;
+        for (int p = warp; p < ps.nprobe; p += nwarps) {
+            const double acc = probe_value(ps, g, p, ts, lane);
+            if (lane == 0) s_val[p] = acc * ps.weight[p];
+        }
+        __syncthreads();
+        for (int k = tid; k < n; k += blockDim.x) {
+            const int p = k / fd.nfreq, f = k - p * fd.nfreq;
+            const double t = ((double)ts + 0.5 * (double)fd.dual[p]) * fd.dT;
+            double sn, cs;
+            sincospi(2.0 * fd.freq[f] * t, &sn, &cs);  // exp(-2 pi i f t) = cs - i sn
+            const double v = s_val[p] * fd.scale;
+            fd.acc[2 * k] += v * cs;
+            fd.acc[2 * k + 1] -= v * sn;
+        }
+        __syncthreads();
+        if (ps.vals) ps.vals += nentry;
     }
-    if (tid == 0) *fd.count += 1;
+    if (tid == 0) *fd.count += count;
 }
 
 // Sum of a pair over a 256-thread block in a fixed order: a shuffle tree in

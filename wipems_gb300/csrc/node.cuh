@@ -93,8 +93,8 @@ struct DevGrid {
 // stores the pair.  Every lane of the warp calls this (act = the lane's node
 // counts: z < Nz-1 and the update ran); `owner` = the segment exists
 // (y < Ny-1, zt < nzt) and this warp is the one that writes it.
-__device__ __forceinline__ void energy_segment(const DevGrid& g, int x, int y, int zt, bool act, bool owner,
-                                               float v0, float v1, float v2, float i0, float i1, float i2) {
+__device__ __forceinline__ void energy_segment_to(float2* eseg, const DevGrid& g, int x, int y, int zt, bool act,
+                                                  bool owner, float v0, float v1, float v2, float i0, float i1, float i2) {
     float pe = 0.f, ph = 0.f;
     if (act) {
         pe = __fadd_rn(__fadd_rn(__fmul_rn(v0, v0), __fmul_rn(v1, v1)), __fmul_rn(v2, v2));
@@ -106,7 +106,12 @@ __device__ __forceinline__ void energy_segment(const DevGrid& g, int x, int y, i
         ph = __fadd_rn(ph, __shfl_down_sync(0xffffffffu, ph, off));
     }
     if (owner && (threadIdx.x & 31) == 0)
-        g.eseg[((long long)x * (g.Ny - 1) + y) * g.nzt + zt] = make_float2(pe, ph);
+        eseg[((long long)x * (g.Ny - 1) + y) * g.nzt + zt] = make_float2(pe, ph);
+}
+
+__device__ __forceinline__ void energy_segment(const DevGrid& g, int x, int y, int zt, bool act, bool owner,
+                                               float v0, float v1, float v2, float i0, float i1, float i2) {
+    energy_segment_to(g.eseg, g, x, y, zt, act, owner, v0, v1, v2, i0, i1, i2);
 }
 
 template <typename IdxT>
@@ -143,6 +148,23 @@ __device__ __forceinline__ GeoF geo_factors(const DevGrid& g, bool H, int x, int
         r.f[n][2] = __ldg(b + p[(n + 2) % 3]);
     }
     return r;
+}
+
+// The excitation of one node, added last in a half-step.
+template <bool H>
+__device__ __forceinline__ void excite_node(const DevGrid& g, float fld[3], uint32_t t, int numTS) {
+    const DevHalf& T = H ? g.h : g.e;
+    const float4 e0 = __ldg(&T.exc[TAB_EXC * t]);
+    const float4 e1 = __ldg(&T.exc[TAB_EXC * t + 1]);
+    const float amp[3] = {e0.x, e0.y, e0.z};
+    const int dly[3] = {__float_as_int(e1.x), __float_as_int(e1.y), __float_as_int(e1.z)};
+    const float* sig = H ? g.sigC : g.sigV;
+#pragma unroll
+    for (int n = 0; n < 3; ++n)
+        if (dly[n] >= 0) {
+            const int k = exc_index(numTS, dly[n], g.sig_len, g.sig_period);
+            fld[n] = __fadd_rn(fld[n], __fmul_rn(amp[n], sig[k]));
+        }
 }
 
 // One node of one half-step.  fld[3]: the old field (V or I); curl[3]: the
@@ -280,19 +302,7 @@ __device__ __forceinline__ void update_node(const DevGrid& g, float fld[3], cons
             for (int n = 0; n < 3; ++n) fld[n] = __fsub_rn(fld[n], Ax[(long long)k * 3 * C + n * C + o]);
         }
     }
-    if (flags & TF_EXC) {
-        const float4 e0 = __ldg(&T.exc[TAB_EXC * t]);
-        const float4 e1 = __ldg(&T.exc[TAB_EXC * t + 1]);
-        const float amp[3] = {e0.x, e0.y, e0.z};
-        const int dly[3] = {__float_as_int(e1.x), __float_as_int(e1.y), __float_as_int(e1.z)};
-        const float* sig = H ? g.sigC : g.sigV;
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
-            if (dly[n] >= 0) {
-                const int k = exc_index(numTS, dly[n], g.sig_len, g.sig_period);
-                fld[n] = __fadd_rn(fld[n], __fmul_rn(amp[n], sig[k]));
-            }
-    }
+    if (flags & TF_EXC) excite_node<H>(g, fld, t, numTS);
 }
 
 }  // namespace wipems
