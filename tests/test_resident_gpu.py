@@ -2,27 +2,37 @@
 fields, samples, energies and frequency-domain sums must equal the direct
 kernels bit for bit, at extents around the 32-node segments and the box
 cuts, with and without UPML, trimmed and untrimmed last lines, graded
-meshes, and through split runs, field writes and restores."""
+meshes, Mur faces, lumped RLC, Drude and Lorentz bricks, and through split runs, field writes and restores."""
 import numpy as np
 import pytest
 
 from wipems_gb300 import CompressedOperator, Engine, Operator, Scene
-from wipems_gb300.fdtd import BC_PEC, BC_PMC, BC_PML
+from wipems_gb300.fdtd import BC_MUR, BC_PEC, BC_PMC, BC_PML
 
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("libs")]
 
 
-def _op(n, wall=BC_PEC, graded=False):
+def _op(n, wall=BC_PEC, graded=False, media=()):
     rng = np.random.default_rng(sum(n))
     lines = [np.cumsum(rng.uniform(0.8, 1.2, k)) if graded else np.arange(k, dtype=float) for k in n]
     s = Scene(*lines, 1e-3)
-    s.set_boundary([wall] * 6, [4] * 6 if wall == BC_PML else [0] * 6)
+    walls = wall if isinstance(wall, list) else [wall] * 6
+    s.set_boundary(walls, [4 if w == BC_PML else 0 for w in walls])
     s.set_gauss_excite(20e9, 20e9, 300)
     c = [k // 2 for k in n]
     at = lambda *i: [lines[a][min(i[a], n[a] - 1)] for a in range(3)]
     s.add_excitation(at(*c), at(c[0], c[1], c[2] + 1), [0.3, 0.0, 1.0])
     if min(n) > 8:
         s.add_material(at(c[0] - 2, c[1] - 3, 5), at(c[0] + 2, c[1] + 1, c[2] + 2), eps_r=3.0, kappa=0.2, priority=10)
+    if "rlc" in media:
+        for k in range(2):
+            s.add_lumped_rlc(at(c[0] - 3, c[1] + 2 + k, c[2]), at(c[0] - 3, c[1] + 2 + k, c[2] + 1), 2, R=50.0, L=2e-9,
+                             Cap=0.5e-12, series=False, caps=False, priority=1000)
+    for k, m in enumerate(("drude", "lorentz")):
+        if m in media:
+            s.add_lorentz(at(c[0] + 1, 3, 4 + 6 * k), at(c[0] + 4, c[1] - 4, 9 + 6 * k), eps_r=2.0, plasma_f=[9e9],
+                          relax_t=[1e-9], pole_f=[6e9 if k else 0.0], mue_plasma_f=[5e9], mue_relax_t=[1e-9],
+                          priority=20 + k)
     s.add_probe(at(c[0], c[1], 0), at(c[0], c[1], n[2] - 1), 0)
     return Operator(s)
 
@@ -33,12 +43,19 @@ def _same(a, b):
         assert x.tobytes() == y.tobytes()
 
 
-@pytest.mark.parametrize("n,wall,graded", [
-    ((3, 3, 3), BC_PEC, False), ((2, 9, 40), BC_PEC, False), ((6, 35, 2), BC_PMC, False),
-    ((33, 9, 65), BC_PMC, False), ((34, 33, 97), BC_PEC, True), ((20, 21, 22), BC_PML, False),
-    ((41, 33, 64), BC_PML, False), ((30, 29, 35), BC_PML, True), ((104, 100, 98), BC_PEC, False)])
-def test_resident_equals_direct(n, wall, graded):
-    cop = CompressedOperator(_op(n, wall, graded))
+_MIX = [BC_MUR, BC_MUR, BC_PEC, BC_MUR, BC_MUR, BC_PMC]
+
+
+@pytest.mark.parametrize("n,wall,graded,media", [
+    ((3, 3, 3), BC_PEC, False, ()), ((2, 9, 40), BC_PEC, False, ()), ((6, 35, 2), BC_PMC, False, ()),
+    ((33, 9, 65), BC_PMC, False, ()), ((34, 33, 97), BC_PEC, True, ()), ((20, 21, 22), BC_PML, False, ()),
+    ((41, 33, 64), BC_PML, False, ()), ((30, 29, 35), BC_PML, True, ()), ((104, 100, 98), BC_PEC, False, ()),
+    ((33, 34, 35), BC_MUR, False, ()), ((22, 31, 65), _MIX, False, ("rlc",)), ((40, 25, 33), BC_MUR, True, ("rlc",)),
+    ((21, 22, 40), BC_PML, False, ("rlc",)), ((30, 26, 37), BC_MUR, False, ("drude",)),
+    ((30, 27, 64), _MIX, False, ("drude", "lorentz")), ((29, 28, 36), BC_PML, False, ("drude", "lorentz")),
+    ((28, 30, 33), BC_PEC, False, ("lorentz", "rlc"))])
+def test_resident_equals_direct(n, wall, graded, media):
+    cop = CompressedOperator(_op(n, wall, graded, media))
     a, b = Engine(cop, max_timesteps=300), Engine(cop, max_timesteps=300, kernel="direct")
     if n[0] < 50:
         for e in (a, b):

@@ -506,12 +506,11 @@ int upload_half(fdtd_engine_s* e, const HalfTables& T, DevHalfBufs& B, DevHalf& 
 
 // Whether runs of timesteps may stay in shared memory (if the grid fits, see
 // setup_resident): the default kernel choice with the default tiling
-// (explicit tilings are the half-step kernels'), 16-bit indices, no
-// Lorentz/Drude nodes, no passes between the half-steps (Mur faces, lumped RLC edges), and no end criterion
-// (which is decided sample by sample).
+// (explicit tilings are the half-step kernels'), 16-bit indices, and no end
+// criterion (which is decided sample by sample).
 bool resident_applies(const fdtd_engine_s* e, const fdtd_cop_s* c, const fdtd_engine_opts* o) {
     if (o && (o->kernel != 0 || o->tile_y > 0 || o->x_chunk > 0 || o->stages > 0)) return false;
-    return c->E.idx16 && c->H.idx16 && !(e->feat & (FEAT_ADE | FEAT_ADEX)) && c->mur.empty() && !c->rlc.size() && e->end_crit == 0.0;
+    return c->E.idx16 && c->H.idx16 && e->end_crit == 0.0;
 }
 
 int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine_s* e) {

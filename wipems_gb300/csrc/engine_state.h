@@ -227,7 +227,7 @@ inline int auto_x_chunk(const std::vector<const uint32_t*>& lines, uint64_t resi
 
 // resident.cu
 // boxes per axis, at most `blocks` of at most `nodes`; false if the grid does not fit
-bool resident_plan(const int cov[3], int blocks, int nodes, int p[3]);
+bool resident_plan(const int cov[3], const bool mur[3], int blocks, int nodes, int p[3]);
 int setup_resident(fdtd_engine_s* e);                    // sets e->resident if the grid fits
 uint32_t resident_run(const fdtd_engine_s* e, uint32_t n);  // timesteps the next launch can take, at most n
 int launch_resident(fdtd_engine_s* e, uint32_t n);       // n timesteps and their samples

@@ -565,34 +565,40 @@ struct RlcSet {
     float* state;          // [7][count]: Il, Vd[3 slots], J[3 slots]
 };
 
+// One edge at numTS: v is the updated voltage, the result its final value.
+__device__ __forceinline__ float rlc_edge(const RlcSet& rs, uint32_t k, int numTS, float v) {
+    const uint32_t n = rs.count;
+    const uint32_t s0 = (uint32_t)(numTS % 3), s1 = (uint32_t)((numTS + 2) % 3), s2 = (uint32_t)((numTS + 1) % 3);
+    const float* c = rs.coef + k;
+    const float ilv = c[0], i2v = c[n], vv2 = c[2 * n], vj1 = c[3 * n], vj2 = c[4 * n], vvd = c[5 * n], ib0 = c[6 * n],
+                b1 = c[7 * n], b2 = c[8 * n];
+    float* Il = rs.state + k;
+    float* Vd = rs.state + n + k;
+    float* J = rs.state + 4 * n + k;
+    // DoPreVoltageUpdates: Il += i2v * ilv * Vd[n-1]
+    const float il = __fadd_rn(Il[0], __fmul_rn(__fmul_rn(i2v, ilv), Vd[s1 * n]));
+    Il[0] = il;
+    const float vd2 = Vd[s2 * n], j1 = J[s1 * n], j2 = J[s2 * n];
+    // Apply2Voltages
+    float t = __fsub_rn(v, il);
+    t = __fadd_rn(t, __fmul_rn(vv2, vd2));
+    t = __fadd_rn(t, __fmul_rn(vj1, j1));
+    t = __fadd_rn(t, __fmul_rn(vj2, j2));
+    const float vd = __fmul_rn(vvd, t);
+    float jn = __fmul_rn(ib0, __fsub_rn(vd, vd2));
+    jn = __fsub_rn(jn, __fmul_rn(__fmul_rn(b1, ib0), j1));
+    jn = __fsub_rn(jn, __fmul_rn(__fmul_rn(b2, ib0), j2));
+    Vd[s0 * n] = vd;
+    J[s0 * n] = jn;
+    return vd;
+}
+
 static __global__ void k_rlc(const DevGrid g, RlcSet rs, int ts_off) {
     if (*g.d_done) return;
     const int numTS = *g.d_ts + ts_off;
-    const uint32_t n = rs.count;
-    const uint32_t s0 = (uint32_t)(numTS % 3), s1 = (uint32_t)((numTS + 2) % 3), s2 = (uint32_t)((numTS + 1) % 3);
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const float* c = rs.coef + k;
-        const float ilv = c[0], i2v = c[n], vv2 = c[2 * n], vj1 = c[3 * n], vj2 = c[4 * n], vvd = c[5 * n],
-                    ib0 = c[6 * n], b1 = c[7 * n], b2 = c[8 * n];
-        float* Il = rs.state + k;
-        float* Vd = rs.state + n + k;
-        float* J = rs.state + 4 * n + k;
-        // DoPreVoltageUpdates: Il += i2v * ilv * Vd[n-1]
-        const float il = __fadd_rn(Il[0], __fmul_rn(__fmul_rn(i2v, ilv), Vd[s1 * n]));
-        Il[0] = il;
-        const float vd2 = Vd[s2 * n], j1 = J[s1 * n], j2 = J[s2 * n];
-        // Apply2Voltages
-        float t = __fsub_rn(g.V[rs.off[k]], il);
-        t = __fadd_rn(t, __fmul_rn(vv2, vd2));
-        t = __fadd_rn(t, __fmul_rn(vj1, j1));
-        t = __fadd_rn(t, __fmul_rn(vj2, j2));
-        const float vd = __fmul_rn(vvd, t);
-        float jn = __fmul_rn(ib0, __fsub_rn(vd, vd2));
-        jn = __fsub_rn(jn, __fmul_rn(__fmul_rn(b1, ib0), j1));
-        jn = __fsub_rn(jn, __fmul_rn(__fmul_rn(b2, ib0), j2));
-        Vd[s0 * n] = vd;
-        J[s0 * n] = jn;
-        g.V[rs.off[k]] = vd;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < rs.count; k += gridDim.x * blockDim.x) {
+        float* v = g.V + rs.off[k];
+        *v = rlc_edge(rs, k, numTS, *v);
     }
 }
 

@@ -21,9 +21,10 @@
 //   41^3 PEC 7.3 -> 2.8                 61^3 UPML 12.1 -> 5.0
 //   65^3 PEC 8.6 -> 4.3                 81^3 UPML 17.8 -> 11.0
 //   91^3 PEC 13.7 -> 9.9                98 x 76 x 132 PEC 16.1 -> 13.3
-//   102^3 PEC 18.9 -> 15.1
-// so every grid that fits runs resident.  Lorentz/Drude states do not fit
-// beside the fields (from global memory: 85 x 77 x 93 multipole 25 -> 35 us).
+//   102^3 PEC 18.9 -> 15.1              61 x 51 x 71 UPML + RLC 13.8 -> 6.3
+//   51 x 42 x 61 Mur 17.3 -> 4.2        91 x 92 x 90 Mur 25.0 -> 10.1
+//   21 x 4 x 1001 Mur, Drude 16.0 -> 3.9 (five launches per timestep before)
+// so every grid that fits runs resident.
 //
 // Arithmetic: as update_node (node.cuh).
 #pragma once
@@ -38,11 +39,21 @@ namespace wipems {
 constexpr int RES_THREADS = 640;   // 96 registers a thread: 768 threads spill
 constexpr int RES_TASKS = 320;     // 32-node tasks of a box
 constexpr int RES_ENTRIES = 512;   // probe entries whose samples are taken inside the run
-// Shared memory of a box of up to NS nodes: the field components (and UPML
-// fluxes) at a constant stride, so that a node's 13 reads share four address
-// registers, the two tuple indices, the task tables, the probe entries.
-__host__ __device__ constexpr int res_smem(int ns, bool upml) {
-    return ns * ((upml ? 12 : 6) * 4 + 2 * 2) + 2 * RES_TASKS * 16 + RES_ENTRIES * 8;
+// Field components a box keeps: V and I, the UPML fluxes, the Drude states
+// and, with RES_LOR, the Lorentz states.
+constexpr int RES_LOR = 256;  // beside the FEAT_ bits
+__host__ __device__ constexpr int res_comps(int feat) {
+    return 6 + ((feat & FEAT_UPML) ? 6 : 0) + ((feat & FEAT_ADE) ? 6 : 0) + ((feat & RES_LOR) ? 6 : 0);
+}
+// Shared memory of a box of up to NS nodes: the components at a constant
+// stride, so that a node's 13 reads share four address registers, the two
+// tuple indices, the task tables, the probe entries and, for runs with passes
+// after the voltage update, the Mur face nodes of the box (four values and
+// two words each) and its lumped RLC edges.
+constexpr int RES_MUR = 2048;
+constexpr int RES_RLC = 128;
+__host__ __device__ constexpr int res_smem(int ns, int feat, bool late) {
+    return ns * (res_comps(feat) * 4 + 2 * 2) + 2 * RES_TASKS * 16 + RES_ENTRIES * 8 + (late ? RES_MUR * 24 + RES_RLC * 8 : 0);
 }
 constexpr unsigned long long RES_WAIT_CYCLES = 4000000000ull;  // ~2 s
 
@@ -50,7 +61,7 @@ constexpr unsigned long long RES_WAIT_CYCLES = 4000000000ull;  // ~2 s
 // box's first node, x | y << 16, z}
 constexpr uint32_t RT_X = 1u << 16;     // the x neighbour (E: x-1, H: x+1) is in the box
 constexpr uint32_t RT_Y = 2u << 16;
-constexpr uint32_t RT_ROW = 16u << 16;  // H: currents live on this row
+constexpr uint32_t RT_ROW = 16u << 16;  // this half-step updates the row
 constexpr uint32_t RT_Z = 32u << 16;    // E: node z-1 of lane 0 is in the box
 
 struct ResArgs {
@@ -67,6 +78,8 @@ struct ResArgs {
     int fd_interval;         // frequency-domain steps: every fd_interval-th timestep (0 = none)
     float* fdval;            // probe entry values per frequency-domain step of the run
     int nentry;
+    MurSet mur;              // Mur faces (nface 0 = none)
+    RlcSet rlc;              // lumped RLC edges (count 0 = none)
     int* d_err;
 };
 
@@ -105,23 +118,44 @@ __device__ __forceinline__ void ll_wait(const ulonglong2* w, uint32_t tag, float
         }
 }
 
-// update_node's arithmetic for the features kept resident; F: the node's
-// UPML flux in shared memory (component stride NS).
-template <bool H, bool UPML, bool GEO, int NS>
+// update_node's arithmetic and order on shared-memory states (component
+// stride NS): F the node's UPML flux, A and L its Lorentz/Drude states.
+template <bool H, int FEAT, bool GEO, int NS>
 __device__ __forceinline__ void res_update(const DevGrid& g, float fld[3], const float curl[3], uint32_t t, float* F,
-                                           int numTS, const GeoF& gf) {
+                                           float* A, float* L, int numTS, const GeoF& gf) {
     const DevHalf& T = H ? g.h : g.e;
     const float4 ta = __ldg(&T.main[TAB_MAIN * t]);
     const float4 tb = __ldg(&T.main[TAB_MAIN * t + 1]);
     const float c1[3] = {ta.x, ta.y, ta.z};
     float c2[3] = {ta.w, tb.x, tb.y};
     const uint32_t flags = __float_as_uint(tb.z);
+    float ade[3];
+    if ((FEAT & FEAT_ADE) && (flags & TF_ADE)) {
+        const float4 a0 = __ldg(&T.ade[TAB_ADE * t]);
+        const float4 a1 = __ldg(&T.ade[TAB_ADE * t + 1]);
+        const float4 a2 = __ldg(&T.ade[TAB_ADE * t + 2]);
+        const float kint[3] = {a0.x, a0.y, a0.z};
+        const float kext[3] = {a0.w, a1.x, a1.y};
+        const float klor[3] = {a1.z, a1.w, a2.x};
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+            float a = A[n * NS], f = fld[n];
+            if ((FEAT & RES_LOR) && (flags & TF_LOR)) {
+                const float l = __fadd_rn(L[n * NS], __fmul_rn(klor[n], a));
+                L[n * NS] = l;
+                f = __fsub_rn(f, l);
+            }
+            a = __fadd_rn(__fmul_rn(a, kint[n]), __fmul_rn(kext[n], f));
+            A[n * NS] = a;
+            ade[n] = a;
+        }
+    }
 #pragma unroll
     for (int n = 0; n < 3; ++n) {
         if (GEO) c2[n] = __fmul_rn(__fmul_rn(__fmul_rn(c2[n], gf.f[n][0]), gf.f[n][1]), gf.f[n][2]);
         c2[n] = __fmul_rn(c2[n], curl[n]);
     }
-    if (UPML && (flags & TF_UPML)) {
+    if ((FEAT & FEAT_UPML) && (flags & TF_UPML)) {
         const float4 u0 = __ldg(&T.upml[TAB_UPML * t]);
         const float4 u1 = __ldg(&T.upml[TAB_UPML * t + 1]);
         const float4 u2 = __ldg(&T.upml[TAB_UPML * t + 2]);
@@ -140,18 +174,159 @@ __device__ __forceinline__ void res_update(const DevGrid& g, float fld[3], const
 #pragma unroll
         for (int n = 0; n < 3; ++n) fld[n] = __fadd_rn(__fmul_rn(fld[n], c1[n]), c2[n]);
     }
+    if ((FEAT & FEAT_ADE) && (flags & TF_ADE)) {
+#pragma unroll
+        for (int n = 0; n < 3; ++n) fld[n] = __fsub_rn(fld[n], ade[n]);
+    }
     if (flags & TF_EXC) excite_node<H>(g, fld, t, numTS);
 }
 
-template <int NS, bool UPML, bool GEO>
+// Engine_Ext_Mur_ABC on the faces of one box: the three passes of k_mur on
+// the voltages in shared memory.  Both lines of a face lie in the box (the
+// plan cuts no axis with a Mur face into boxes of one line).  Everything that
+// does not change is put into a list once, so a pass is a few instructions
+// per face node; the same thread takes a node in every pass.
+//   node: .x = slot on the face | slot of the next line << 13 | normal axis
+//              << 26 | face << 28 | counts as zero << 31
+//         .y = earlier faces that would write component n+1 (6 bits), n+2 (6
+//              bits), excitation << 12, tuple << 16
+//   val: {cp, cpp, bp, bpp}
+template <int NS>
+struct ResMur {
+    float* sV;
+    uint2* node;
+    float4* val;
+    int count;  // of this box
+
+    __device__ __forceinline__ void init(const DevGrid& g, const MurSet& ms, float* v, const uint16_t* sE, float4* vals,
+                                         uint2* nodes, int lx, int ly, int lz, int bx, int by, int bz) {
+        sV = v;
+        val = vals;
+        node = nodes;
+        count = 0;
+        const int Nl[3] = {g.Nx - 1, g.Ny - 1, g.Nz - 1};
+        for (int fi = 0; fi < ms.nface; ++fi) {
+            const MurDev F = ms.f[fi];
+            const int ny = F.ny;
+            const int l0 = ny == 0 ? lx : ny == 1 ? ly : lz, n0 = ny == 0 ? bx : ny == 1 ? by : bz;  // along the normal
+            const int lP = ny == 0 ? ly : ny == 1 ? lz : lx, nP = ny == 0 ? by : ny == 1 ? bz : bx;
+            const int lQ = ny == 0 ? lz : ny == 1 ? lx : ly, nQ = ny == 0 ? bz : ny == 1 ? bx : by;
+            if (F.line < l0 || F.line >= l0 + n0) continue;
+            for (int q = threadIdx.x; q < nP * nQ; q += blockDim.x) {
+                const int i = q / nQ, j = q - i * nQ;
+                auto slot = [&](int line) {
+                    const int x = ny == 0 ? line : ny == 1 ? j : i, y = ny == 0 ? i : ny == 1 ? line : j,
+                              z = ny == 0 ? j : ny == 1 ? i : line;
+                    return (uint32_t)((x * by + y) * bz + z);
+                };
+                const uint32_t ol = slot(F.line - l0), os = slot(F.shift - l0);
+                const int X = ny == 0 ? F.line : ny == 1 ? j + lx : i + lx, Y = ny == 0 ? i + ly : ny == 1 ? F.line : j + ly,
+                          Z = ny == 0 ? j + lz : ny == 1 ? i + lz : F.line;
+                uint32_t m1 = 0, m2 = 0;
+                for (int e = 0; e < fi; ++e) {
+                    const int gn = ms.f[e].ny, p = gn == 0 ? X : gn == 1 ? Y : Z;
+                    if (p != ms.f[e].line) continue;
+                    if (gn != (ny + 1) % 3) m1 |= 1u << e;
+                    if (gn != (ny + 2) % 3) m2 |= 1u << e;
+                }
+                // a last line that the voltage update leaves out counts as zero
+                const int P = ny == 0 ? 1 : ny == 1 ? 2 : 0, Q = ny == 0 ? 2 : ny == 1 ? 0 : 1;
+                const bool inert = (ms.trim[P] && i + lP == Nl[P]) || (ms.trim[Q] && j + lQ == Nl[Q]);
+                const uint32_t t = sE[ol];
+                const bool exc = __float_as_uint(__ldg(&g.e.main[TAB_MAIN * t + 1]).z) & TF_EXC;
+                const int loc = (i + lP) * F.n1 + j + lQ;
+                node[count + q] = make_uint2(ol | os << 13 | (uint32_t)ny << 26 | (uint32_t)fi << 28 | (inert ? 1u << 31 : 0u),
+                                             m1 | m2 << 6 | (exc ? 1u << 12 : 0u) | t << 16);
+                val[count + q] = make_float4(F.cp[loc], F.cpp[loc], F.bp[loc], F.bpp[loc]);
+            }
+            count += nP * nQ;
+        }
+    }
+    // faces that act at numTS ts
+    static __device__ __forceinline__ uint32_t active(const MurSet& ms, int ts) {
+        uint32_t m = 0;
+        for (int fi = 0; fi < ms.nface; ++fi) m |= ts >= ms.f[fi].start_ts ? 1u << fi : 0u;
+        return m;
+    }
+    static __device__ __forceinline__ int comp(int n) { return n >= 3 ? (n - 3) * NS : n * NS; }
+    __device__ __forceinline__ void pre(uint32_t act) const {
+        for (int q = threadIdx.x; q < count; q += blockDim.x) {
+            const uint32_t e = node[q].x;
+            if (!(act >> (e >> 28 & 7u) & 1u)) continue;
+            const int ol = e & 8191u, os = e >> 13 & 8191u, ny = e >> 26 & 3u;
+            const float* vP = sV + comp(ny + 1);
+            const float* vQ = sV + comp(ny + 2);
+            float4 w = val[q];
+            w.z = __fsub_rn(vP[os], __fmul_rn(w.x, vP[ol]));
+            w.w = __fsub_rn(vQ[os], __fmul_rn(w.y, vQ[ol]));
+            val[q] = w;
+        }
+    }
+    __device__ __forceinline__ void post(uint32_t act) const {
+        for (int q = threadIdx.x; q < count; q += blockDim.x) {
+            const uint32_t e = node[q].x;
+            if (!(act >> (e >> 28 & 7u) & 1u)) continue;
+            const int os = e >> 13 & 8191u, ny = e >> 26 & 3u;
+            const bool zero = e >> 31;
+            float4 w = val[q];
+            w.z = __fadd_rn(w.z, __fmul_rn(w.x, zero ? 0.f : sV[comp(ny + 1) + os]));
+            w.w = __fadd_rn(w.w, __fmul_rn(w.y, zero ? 0.f : sV[comp(ny + 2) + os]));
+            val[q] = w;
+        }
+    }
+    __device__ __forceinline__ void apply(const DevGrid& g, uint32_t act, int ts) const {
+        for (int q = threadIdx.x; q < count; q += blockDim.x) {
+            const uint2 e = node[q];
+            if (!(act >> (e.x >> 28 & 7u) & 1u)) continue;
+            const int ol = e.x & 8191u, ny = e.x >> 26 & 3u;
+            const float4 w = val[q];
+            float v1 = w.z, v2 = w.w;
+            if (e.y & 1u << 12) {
+                float v[3] = {ny == 0 ? 0.f : ny == 1 ? v2 : v1, ny == 0 ? v1 : ny == 1 ? 0.f : v2,
+                              ny == 0 ? v2 : ny == 1 ? v1 : 0.f};
+                excite_node<false>(g, v, e.y >> 16, ts);
+                v1 = ny == 0 ? v[1] : ny == 1 ? v[2] : v[0];
+                v2 = ny == 0 ? v[2] : ny == 1 ? v[0] : v[1];
+            }
+            if (!(e.y & act & 63u)) sV[comp(ny + 1) + ol] = v1;
+            if (!(e.y >> 6 & act & 63u)) sV[comp(ny + 2) + ol] = v2;
+        }
+    }
+    // the values back to the engine's buffers
+    __device__ __forceinline__ void store(const MurSet& ms, int lx, int ly, int lz, int bx, int by, int bz) const {
+        int first = 0;
+        for (int fi = 0; fi < ms.nface; ++fi) {
+            const MurDev F = ms.f[fi];
+            const int ny = F.ny;
+            const int l0 = ny == 0 ? lx : ny == 1 ? ly : lz, n0 = ny == 0 ? bx : ny == 1 ? by : bz;
+            const int lP = ny == 0 ? ly : ny == 1 ? lz : lx, nP = ny == 0 ? by : ny == 1 ? bz : bx;
+            const int lQ = ny == 0 ? lz : ny == 1 ? lx : ly, nQ = ny == 0 ? bz : ny == 1 ? bx : by;
+            if (F.line < l0 || F.line >= l0 + n0) continue;
+            for (int q = threadIdx.x; q < nP * nQ; q += blockDim.x) {
+                const int i = q / nQ, j = q - i * nQ, loc = (i + lP) * F.n1 + j + lQ;
+                F.bp[loc] = val[first + q].z;
+                F.bpp[loc] = val[first + q].w;
+            }
+            first += nP * nQ;
+        }
+    }
+};
+
+// LATE: the grid has Mur faces or lumped RLC edges.
+template <int NS, int FEAT, bool GEO, bool LATE>
 __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const ResArgs a, const ProbeSet ps) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ int s_nent;
-    constexpr int NF = UPML ? 12 : 6;
+    __shared__ int s_nent, s_nrlc;
+    constexpr bool UPML = (FEAT & FEAT_UPML) != 0, ADE = (FEAT & FEAT_ADE) != 0, LOR = (FEAT & RES_LOR) != 0;
+    constexpr int NF = res_comps(FEAT), OA = UPML ? 12 : 6;
     float* const sV = sm;
     float* const sI = sm + 3 * NS;
-    float* const sFV = sm + 6 * NS;  // UPML only
+    float* const sFV = sm + 6 * NS;         // UPML only
     float* const sFI = sm + 9 * NS;
+    float* const sAV = sm + OA * NS;        // Lorentz/Drude only
+    float* const sAI = sm + (OA + 3) * NS;
+    float* const sLV = sm + (OA + 6) * NS;  // Lorentz only
+    float* const sLI = sm + (OA + 9) * NS;
     uint16_t* const sE = reinterpret_cast<uint16_t*>(sm + NF * NS);
     uint16_t* const sH = sE + NS;
     uint4* const tabE = reinterpret_cast<uint4*>(sm + (NF + 1) * NS);
@@ -169,7 +344,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
 
     // The tasks that need no neighbour box come first: what the others wait
     // for travels meanwhile.  A thread places each task by counting.
-    if (tid == 0) s_nent = 0;
+    if (tid == 0) s_nent = s_nrlc = 0;
     auto edgeE = [&](int x, int y, int zc) {
         return (x == 0 && ix > 0) || (y == 0 && iy > 0) || (zc == 0 && iz > 0);
     };
@@ -195,7 +370,8 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
             const int z = zc * 32;
             const uint32_t o = (uint32_t)(r * bz + z), go = (uint32_t)(x * g.sx + (long long)y * g.Nzp + z);
             tabE[edgeE(x, y, zc) ? outE++ : inE++] =
-                make_uint4(o | (x > 0 ? RT_X : 0u) | (y > 0 ? RT_Y : 0u) | (z > 0 ? RT_Z : 0u), go,
+                make_uint4(o | (x > 0 ? RT_X : 0u) | (y > 0 ? RT_Y : 0u) | (z > 0 ? RT_Z : 0u) |
+                               (lx + x < a.ne[0] && ly + y < a.ne[1] ? RT_ROW : 0u), go,
                            (uint32_t)(x | y << 16), (uint32_t)z);
             tabH[edgeH(x, y, zc) ? outH++ : inH++] =
                 make_uint4(o | (x + 1 < bx ? RT_X : 0u) | (y + 1 < by ? RT_Y : 0u) |
@@ -215,6 +391,12 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
                 if (UPML) {
                     sFV[c * NS + o] = g.FV[c * C + go + z];
                     sFI[c * NS + o] = g.FI[c * C + go + z];
+                }
+                if (ADE) {
+                    if (g.AV) sAV[c * NS + o] = g.AV[c * C + go + z];
+                    if (LOR && g.LV) sLV[c * NS + o] = g.LV[c * C + go + z];
+                    if (g.AI) sAI[c * NS + o] = g.AI[c * C + go + z];
+                    if (LOR && g.LI) sLI[c * NS + o] = g.LI[c * C + go + z];
                 }
             }
             sE[o] = (uint16_t)load_idx<uint16_t>(g.e.idx, go + z);
@@ -241,7 +423,33 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
     const int yl = oY + ((iy - 1) * a.cov[0] + lx) * a.cov[2] + lz, yh = yl + a.cov[0] * a.cov[2];
     const int zl = oZ + ((iz - 1) * a.cov[0] + lx) * a.cov[1] + ly, zh = zl + a.cov[0] * a.cov[1];
     const bool hasx = ix + 1 < a.p[0], hasy = iy + 1 < a.p[1], hasz = iz + 1 < a.p[2];
-    const int zH = min(bz, g.Nz - 1 - lz);  // nodes of a row with currents
+    const int zE = min(bz, a.ne[2] - lz), zH = min(bz, g.Nz - 1 - lz);  // nodes of a row each half-step updates
+
+    auto send_volt = [&](const uint4 e, int z, float v0, float v1, float v2, ulonglong2* llV, uint32_t tag) {
+        const int x = (int)(e.z & 0xffffu), y = (int)(e.z >> 16);
+        if (x == 0 && ix > 0) ll_send(llV + (xl + y * a.cov[2] + z), v1, v2, tag);
+        if (y == 0 && iy > 0) ll_send(llV + (yl + x * a.cov[2] + z), v0, v2, tag);
+        if (z == 0 && iz > 0) ll_send(llV + (zl + x * a.cov[1] + y), v0, v1, tag);
+    };
+    // passes after the voltage update, in boxes that have any
+    ResMur<NS> mur;
+    uint2* const rlc = reinterpret_cast<uint2*>(ent + RES_ENTRIES);  // {edge, slot of its voltage}
+    bool late = false;
+    if (LATE) {
+        uint2* const nodes = rlc + RES_RLC;
+        mur.init(g, a.mur, sV, sE, reinterpret_cast<float4*>(nodes + RES_MUR), nodes, lx, ly, lz, bx, by, bz);
+        for (uint32_t q = tid; q < a.rlc.count; q += blockDim.x) {
+            const long long off = a.rlc.off[q];
+            const int c = (int)(off / C), r = (int)((off - c * C) % g.sx);
+            const int x = (int)((off - c * C) / g.sx) - lx, y = r / g.Nzp - ly, z = r % g.Nzp - lz;
+            if (x < 0 || x >= bx || y < 0 || y >= by || z < 0 || z >= bz) continue;
+            rlc[atomicAdd(&s_nrlc, 1)] = make_uint2(q, (uint32_t)(c * NS + (x * by + y) * bz + z));
+        }
+        __syncthreads();
+        late = mur.count || s_nrlc;
+        mur.pre(mur.active(a.mur, a.ts0));
+        __syncthreads();
+    }
 
     bool ok = true;
     int samples = 0, fds = 0;
@@ -289,27 +497,42 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
                     if (nz) ll_wait(llJ + (zl + x * a.cov[1] + y), (uint32_t)ts, i0zm, i1zm, ok);
                 }
             }
+            if (z < zE && (e.x & RT_ROW)) {
             float curl[3];
             curl[0] = __fadd_rn(__fsub_rn(__fsub_rn(c2, i2ym), c1), i1zm);
             curl[1] = __fadd_rn(__fsub_rn(__fsub_rn(c0, i0zm), c2), i2xm);
             curl[2] = __fadd_rn(__fsub_rn(__fsub_rn(c1, i1xm), c0), i0ym);
             GeoF gf;
             if (GEO) gf = geo_factors(g, false, lx + (int)(e.z & 0xffffu), ly + (int)(e.z >> 16), lz + z);
-            res_update<false, UPML, GEO, NS>(g, v, curl, tu, sFV + o, ts, gf);
+            res_update<false, FEAT, GEO, NS>(g, v, curl, tu, sFV + o, sAV + o, sLV + o, ts, gf);
             sV[o] = v[0];
             sV[NS + o] = v[1];
             sV[2 * NS + o] = v[2];
-            if (EDGE) {
-                const int x = (int)(e.z & 0xffffu), y = (int)(e.z >> 16);
-                if (x == 0 && ix > 0) ll_send(llV + (xl + y * a.cov[2] + z), v[1], v[2], tag);
-                if (y == 0 && iy > 0) ll_send(llV + (yl + x * a.cov[2] + z), v[0], v[2], tag);
-                if (z == 0 && iz > 0) ll_send(llV + (zl + x * a.cov[1] + y), v[0], v[1], tag);
             }
+            if (EDGE && !(LATE && late)) send_volt(e, z, v[0], v[1], v[2], llV, tag);
         };
         int t = warp;
         for (; t < ninE; t += nwarps) volt(std::false_type{}, tabE[t]);
         for (; t < ntask; t += nwarps) volt(std::true_type{}, tabE[t]);
         if (__syncthreads_or(!ok)) break;
+        if (LATE && late) {
+            // the hooks around the voltage update in the reference's order:
+            // Mur post-update, lumped RLC, Mur apply; then the new voltages go out
+            const uint32_t act = mur.active(a.mur, ts);
+            mur.post(act);
+            __syncthreads();
+            if (s_nrlc) {
+                for (int q = tid; q < s_nrlc; q += blockDim.x) sm[rlc[q].y] = rlc_edge(a.rlc, rlc[q].x, ts, sm[rlc[q].y]);
+                __syncthreads();
+            }
+            mur.apply(g, act, ts);
+            __syncthreads();
+            for (int q = ninE + warp; q < ntask; q += nwarps) {
+                const uint4 e = tabE[q];
+                const int z = (int)e.w + lane, o = (int)(e.x & 0xffffu) + lane;
+                if (z < bz) send_volt(e, z, sV[o], sV[NS + o], sV[2 * NS + o], llV, tag);
+            }
+        }
         // ------------------------------------------------------- currents
         const bool sample = a.interval > 0 && (ts + 1) % a.interval == 0;
         auto curr = [&](auto edge, const uint4 e) {
@@ -366,7 +589,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
                 curl[2] = __fadd_rn(__fsub_rn(__fsub_rn(c1, v1xp), c0), v0yp);
                 GeoF gf;
                 if (GEO) gf = geo_factors(g, true, lx + (int)(e.z & 0xffffu), ly + (int)(e.z >> 16), lz + z);
-                res_update<true, UPML, GEO, NS>(g, cu, curl, tu, sFI + o, ts, gf);
+                res_update<true, FEAT, GEO, NS>(g, cu, curl, tu, sFI + o, sAI + o, sLI + o, ts, gf);
                 sI[o] = cu[0];
                 sI[NS + o] = cu[1];
                 sI[2 * NS + o] = cu[2];
@@ -387,6 +610,8 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
         t = warp;
         for (; t < ninH; t += nwarps) curr(std::false_type{}, tabH[t]);
         for (; t < ntask; t += nwarps) curr(std::true_type{}, tabH[t]);
+        // the next timestep's Mur pre-update: the voltages stay as they are until then
+        if (LATE && late && k + 1 < a.nsteps) mur.pre(mur.active(a.mur, ts + 1));
         if (__syncthreads_or(!ok)) break;
         const bool fd = a.fd_interval > 0 && (ts + 1) % a.fd_interval == 0;
         if (sample || fd) {
@@ -401,6 +626,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
         }
     }
     if (!ok) atomicOr(a.d_err, 4);
+    if (LATE && late) mur.store(a.mur, lx, ly, lz, bx, by, bz);
     for (int r = warp; r < rows; r += nwarps) {
         const int x = r / by, y = r - x * by;
         const long long go = g0 + (long long)x * g.sx + (long long)y * g.Nzp;
@@ -413,6 +639,12 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
                 if (UPML) {
                     g.FV[c * C + go + z] = sFV[c * NS + o];
                     g.FI[c * C + go + z] = sFI[c * NS + o];
+                }
+                if (ADE) {
+                    if (g.AV) g.AV[c * C + go + z] = sAV[c * NS + o];
+                    if (LOR && g.LV) g.LV[c * C + go + z] = sLV[c * NS + o];
+                    if (g.AI) g.AI[c * C + go + z] = sAI[c * NS + o];
+                    if (LOR && g.LI) g.LI[c * C + go + z] = sLI[c * NS + o];
                 }
             }
         }

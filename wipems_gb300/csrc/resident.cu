@@ -10,19 +10,43 @@
 namespace wipems {
 namespace {
 
-// box capacities compiled; with UPML the fluxes take their share
-constexpr int kNodes[4] = {1536, 3072, 4096, 7680};
-template <int NS, bool UPML>
+// Box capacities compiled: a small box leaves the L1 cache what it does not
+// need (the tuple tables live there); UPML and Lorentz/Drude states and Mur
+// nodes take their share of the largest.  Lorentz/Drude on graded meshes is
+// left to the half-step kernels: thousands of distinct tuples miss L1 on
+// every node (71 x 51 x 61 lines 11.2 against 11.3 us per step).
+template <int NS, int FEAT, bool LATE = false>
 const void* kernel_g(bool geo) {
-    return geo ? (const void*)k_resident<NS, UPML, true> : (const void*)k_resident<NS, UPML, false>;
+    return geo ? (const void*)k_resident<NS, FEAT, true, LATE> : (const void*)k_resident<NS, FEAT, false, LATE>;
 }
-const void* kernel_of(int ns, bool upml, bool geo) {
-    switch (ns) {
-        case kNodes[0]: return upml ? kernel_g<kNodes[0], true>(geo) : kernel_g<kNodes[0], false>(geo);
-        case kNodes[1]: return upml ? kernel_g<kNodes[1], true>(geo) : kernel_g<kNodes[1], false>(geo);
-        case kNodes[2]: return upml ? kernel_g<kNodes[2], true>(geo) : kernel_g<kNodes[2], false>(geo);
-        default: return kernel_g<kNodes[3], false>(geo);
+struct Variant {
+    int ns;  // capacity (0 = no such variant)
+    const void* kernel;
+};
+Variant variant_of(int nodes, int feat, bool geo, bool late) {
+    constexpr int U = FEAT_UPML, A = FEAT_ADE;
+    if (feat == 0 && !late) {
+        if (nodes <= 1536) return {1536, kernel_g<1536, 0>(geo)};
+        if (nodes <= 3072) return {3072, kernel_g<3072, 0>(geo)};
+        return {7680, kernel_g<7680, 0>(geo)};
     }
+    if (feat == U && !late) {
+        if (nodes <= 1536) return {1536, kernel_g<1536, U>(geo)};
+        if (nodes <= 3072) return {3072, kernel_g<3072, U>(geo)};
+        return {4096, kernel_g<4096, U>(geo)};
+    }
+    if (feat == 0) {
+        if (nodes <= 3072) return {3072, kernel_g<3072, 0, true>(geo)};
+        return {5632, kernel_g<5632, 0, true>(geo)};
+    }
+    if (feat == U) return {3072, kernel_g<3072, U, true>(geo)};
+    if (feat == A && !geo) return {3072, late ? (const void*)k_resident<3072, A, false, true>
+                                              : (const void*)k_resident<3072, A, false, false>};
+    if (feat == (A | RES_LOR) && !geo) return {2048, late ? (const void*)k_resident<2048, A | RES_LOR, false, true>
+                                                          : (const void*)k_resident<2048, A | RES_LOR, false, false>};
+    if ((feat & ~RES_LOR) == (A | U) && !geo && !late)
+        return {2048, (const void*)k_resident<2048, A | U | RES_LOR, false, false>};
+    return {0, nullptr};
 }
 
 constexpr size_t kSampleBytes = (size_t)64 << 20;  // of a run's energy segments
@@ -35,7 +59,7 @@ constexpr uint32_t kMaxRun = 1024;  // timesteps of one launch
 // The cut with the cheapest largest box: its 32-node tasks (eight or fewer
 // take the same time), its rows at a cut (which wait for a neighbour), and a
 // z cut's lone lanes.
-bool resident_plan(const int cov[3], int blocks, int nodes, int p[3]) {
+bool resident_plan(const int cov[3], const bool mur[3], int blocks, int nodes, int p[3]) {
     const int segs = (cov[2] + 31) / 32;
     double best = 1e30;
     for (int pz = 1; pz <= std::min(segs, blocks); ++pz) {
@@ -45,6 +69,12 @@ bool resident_plan(const int cov[3], int blocks, int nodes, int p[3]) {
                 const int bx = (cov[0] + px - 1) / px, by = (cov[1] + py - 1) / py, bz = std::min(32 * nzc, cov[2]);
                 const long long tasks = (long long)bx * by * nzc;
                 if ((long long)bx * by * bz > nodes || tasks > RES_TASKS) continue;
+                // a Mur face and the line next to it lie in one box, the face nodes fit
+                if ((mur[0] && cov[0] / px < 2) || (mur[1] && cov[1] / py < 2) ||
+                    (mur[2] && cov[2] - res_cut_z(cov[2], pz, pz - 1) < 2))
+                    continue;
+                auto faces = [&](int k, int q) { return mur[k] ? (q == 1 ? 2 : 1) : 0; };
+                if (faces(0, px) * by * bz + faces(1, py) * bx * bz + faces(2, pz) * bx * by > RES_MUR) continue;
                 const double cost = std::max(8.0, (double)tasks) + 0.25 * (bx + by) * nzc +
                                     (pz > 1 ? 0.1 * bx * by : 0.0) + 1e-3 * (px * py * pz);
                 if (cost < best) {
@@ -66,19 +96,31 @@ int setup_resident(fdtd_engine_s* e) {
     CK(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
     ResArgs& a = e->ra;
     const size_t entries = e->h_entries.size();
-    for (int k = 0; k < 3; ++k) a.cov[k] = a.ne[k] = e->ti.ne[k];
-    const bool up = (e->feat & FEAT_UPML) != 0;
-    if (!coop || entries > RES_ENTRIES || !resident_plan(a.cov, sms, kNodes[up ? 2 : 3], a.p)) return FDTD_OK;
+    // Mur faces change lines that the voltage update leaves out
+    bool mur[3] = {false, false, false};
+    for (int k = 0; k < e->mur.nface; ++k) mur[e->mur.f[k].ny] = true;
+    for (int k = 0; k < 3; ++k) {
+        a.ne[k] = e->ti.ne[k];
+        a.cov[k] = e->mur.nface ? (int)e->N[k] : a.ne[k];
+    }
+    a.mur = e->mur;
+    a.rlc = e->rlc;
+    const bool late = e->mur.nface || e->rlc.count;
+    int feat = e->feat | (e->LV.p || e->LI.p ? RES_LOR : 0);
+    if ((feat & (FEAT_ADE | FEAT_UPML)) == (FEAT_ADE | FEAT_UPML)) feat |= RES_LOR;
+    const int cap = variant_of(1 << 30, feat, e->geo_on, late).ns;
+    if (!coop || cap == 0 || entries > RES_ENTRIES || e->rlc.count > RES_RLC ||
+        !resident_plan(a.cov, mur, sms, cap, a.p))
+        return FDTD_OK;
     const int segs = (a.cov[2] + 31) / 32, nzc = (segs + a.p[2] - 1) / a.p[2];
     const int bx = (a.cov[0] + a.p[0] - 1) / a.p[0], by = (a.cov[1] + a.p[1] - 1) / a.p[1],
               bz = std::min(32 * nzc, a.cov[2]);
-    int ns = kNodes[0];
-    for (int k = 1; k < 4 && bx * by * bz > ns; ++k) ns = kNodes[k];
-    const int need = res_smem(ns, up);
+    const Variant v = variant_of(bx * by * bz, feat, e->geo_on, late);
+    const int need = res_smem(v.ns, feat, late);
     if (smem < need + 64) return FDTD_OK;
     e->res_smem = need;
     e->res_threads = 32 * std::min(RES_THREADS / 32, bx * by * nzc);
-    e->res_kernel = kernel_of(ns, up, e->geo_on);
+    e->res_kernel = v.kernel;
     CK(cudaFuncSetAttribute(e->res_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, need));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, e->res_kernel, e->res_threads, (size_t)need));
