@@ -264,6 +264,7 @@ struct fdtd_batch_s {
     uint32_t graph_steps = 8;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_jobs = nullptr;     // orders a run after the jobs' own streams
     double last_ms = 0;
     uint64_t last_launches = 0;
     uint64_t device_bytes = 0;
@@ -272,6 +273,7 @@ struct fdtd_batch_s {
         if (graph) cudaGraphExecDestroy(graph);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
+        if (ev_jobs) cudaEventDestroy(ev_jobs);
         for (cudaEvent_t e : ev_fork) cudaEventDestroy(e);
         for (cudaEvent_t e : ev_join) cudaEventDestroy(e);
         for (cudaStream_t s : side) cudaStreamDestroy(s);
@@ -390,6 +392,7 @@ int build_batch(const fdtd_engine_t* engines, uint32_t n, const fdtd_batch_opts*
     CK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&b->ev0));
     CK(cudaEventCreate(&b->ev1));
+    CK(cudaEventCreateWithFlags(&b->ev_jobs, cudaEventDisableTiming));
     int rc;
     for (uint32_t j = 0; j < n; ++j) {
         fdtd_engine_s* e = engines[j];
@@ -631,6 +634,11 @@ int fdtd_batch_iterate(fdtd_batch_t b, uint32_t n) {
     b->last_launches = 0;
     int rc;
     if (b->graph_steps > 1 && n >= b->graph_steps && (rc = batch_graph(b))) return rc;
+    // what the jobs' own streams still hold (a reset, say) comes first
+    for (fdtd_engine_s* e : b->jobs) {
+        CK(cudaEventRecord(b->ev_jobs, e->stream));
+        CK(cudaStreamWaitEvent(b->stream, b->ev_jobs, 0));
+    }
     CK(cudaEventRecord(b->ev0, b->stream));
     uint32_t left = n;
     while (left > 0) {
