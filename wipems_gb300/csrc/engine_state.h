@@ -202,20 +202,29 @@ struct fdtd_engine_s {
 
 
 namespace wipems {
-// x-chunk (planes per block: 1, 2, 4, 8 or 16) from a wave model of the
-// current-kernel grid: a block costs about (2 + x_chunk) plane times (the
-// ring prologue, then one plane each), blocks run in waves of `resident`,
-// so the step costs ceil(blocks / resident) * (2 + x_chunk); a chunk that
-// leaves SMs idle in the only wave is skipped, ties go to the longer chunk
-// (fewer halo-plane re-reads).  lines: the jobs' (Nx, Ny, Nz) triples.
-inline int auto_x_chunk(const std::vector<const uint32_t*>& lines, uint64_t resident, int ty = TMA_TY) {
+// x-chunk (planes per block) from a wave model of the current-kernel grid: a
+// block costs about (2 + x_chunk) plane times (the ring prologue, then one
+// plane each), blocks run in waves of `resident`, so the step costs
+// ceil(blocks / resident) * (2 + x_chunk); a chunk that leaves SMs idle in the
+// only wave is skipped, ties go to the longer chunk (fewer halo-plane
+// re-reads).  lines: the jobs' (Nx, Ny, Nz) triples.  `single`: one job on
+// the half-step kernels, whose chunks are 1, 2 or 4 planes, or 6 with eight
+// waves to spare: longer ones end the voltage half-step far from where the
+// current one starts, and what it left in L2 is gone (257^3 UPML 16 planes
+// 266 us per step, 8: 261, 6: 256, 4: 260; 161^3 UPML 8: 88, 6: 83, 4: 81.6;
+// 257^3 PEC 16: 202, 6 and 4: 194).  Otherwise 1, 2, 4, 8 or 16.
+inline int auto_x_chunk(const std::vector<const uint32_t*>& lines, uint64_t resident, int ty = TMA_TY,
+                        bool single = false) {
     int best = 1;
     uint64_t best_cost = ~0ull;
-    for (int xc = 16; xc >= 1; xc /= 2) {
+    static const int own[] = {6, 4, 2, 1}, shared[] = {16, 8, 4, 2, 1};
+    for (int k = 0; k < (single ? 4 : 5); ++k) {
+        const int xc = single ? own[k] : shared[k];
         uint64_t items = 0;
         for (const uint32_t* N : lines)
             items += (uint64_t)((N[2] - 1 + 31) / 32) * ((N[1] - 1 + ty - 1) / ty) * ((N[0] - 1 + xc - 1) / xc);
         if (items < resident && xc > 1) continue;
+        if (xc == 6 && items < 8 * resident) continue;
         const uint64_t cost = (items + resident - 1) / resident * (uint64_t)(2 + xc);
         if (cost < best_cost) {
             best_cost = cost;
