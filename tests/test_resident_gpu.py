@@ -6,7 +6,7 @@ meshes, Mur faces, lumped RLC, Drude and Lorentz bricks, and through split runs,
 import numpy as np
 import pytest
 
-from wipems_gb300 import CompressedOperator, Engine, Operator, Scene
+from wipems_gb300 import Batch, CompressedOperator, Engine, Operator, Scene
 from wipems_gb300.fdtd import BC_MUR, BC_PEC, BC_PMC, BC_PML
 
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("libs")]
@@ -89,3 +89,23 @@ def test_resident_writes_and_restore():
         e.reset()
         e.iterate(45)
     _same(a, b)
+
+
+@pytest.mark.parametrize("sizes", [[(20, 21, 22)] * 3, [(104, 100, 98), (130, 128, 120), (30, 31, 33)]])
+def test_batch_jobs_outside_the_batched_kernels(sizes):
+    """Batches whose jobs run resident or on their own kernels: the same
+    samples (none before the first timestep of a batch after a reset) and
+    fields as L2 bins, which keep every job in the batched kernels."""
+    cops = [CompressedOperator(_op(n, BC_PML if k % 2 else BC_PEC)) for k, n in enumerate(sizes)]
+    out = []
+    for kw in (dict(x_chunk=64, blocks_per_sm=-1, chains=2), dict(bin_mib=64)):
+        es = [Engine(c, max_timesteps=300, kernel="tma") for c in cops]
+        b = Batch(es, graph_steps=8, **kw)
+        b.iterate(21)
+        for e in es:
+            e.reset()
+        b.iterate(50)
+        out.append(es)
+    for x, y in zip(*out):
+        assert x.num_timesteps == y.num_timesteps == 50
+        _same(x, y)

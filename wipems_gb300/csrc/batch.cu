@@ -17,6 +17,8 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <array>
+#include <set>
 #include <tuple>
 #include <vector>
 
@@ -193,6 +195,55 @@ int batch_smem_attrs(int bytes) {
     return FDTD_OK;
 }
 
+// How long a timestep of a job, or of a set of batched jobs, takes (us), from
+// measurements: a resident job 41^3 PEC 2.8, 65^3 4.3, 91^3 9.9, 61^3 UPML
+// 5.0, 81^3 11.0; a job on its own half-step kernels 98 x 76 x 132 PEC 16.1,
+// 257^3 194, 119 x 102 x 151 UPML 38, 161^3 82; a batch the larger of its
+// longest x-chunk (8 x 41^3 PEC 49, 8 x 65^3 71, 8 x 41^3 UPML 85, 8 x 61^3
+// 138) and its throughput (96 jobs of a million nodes: 58 nodes per ns).
+double nodes_of(const fdtd_engine_s* e) { return (double)e->N[0] * e->N[1] * e->N[2]; }
+bool upml(const fdtd_engine_s* e) { return (e->feat & FEAT_UPML) != 0; }
+double resident_us(const fdtd_engine_s* e) {
+    return upml(e) ? 2.2 + 16.5e-6 * nodes_of(e) : 1.9 + 11.3e-6 * nodes_of(e);
+}
+double own_us(const fdtd_engine_s* e) { return upml(e) ? 5.0 + 19e-6 * nodes_of(e) : 4.0 + 12.5e-6 * nodes_of(e); }
+double batched_us(const std::vector<fdtd_engine_s*>& jobs, int XC) {
+    double longest = 0.0, nodes = 0.0;
+    for (const fdtd_engine_s* e : jobs) {
+        const int planes = XC > 0 ? std::min(XC, (int)e->N[0]) : std::min(16, (int)e->N[0]);
+        longest = std::max(longest, (upml(e) ? 2.2 : 1.1) * planes);
+        nodes += nodes_of(e);
+    }
+    return std::max(longest, nodes / 58e3);
+}
+
+// Which jobs leave the batched kernels: those that run resident
+// (kernels_resident.cuh), if together, or else one by one, that is the faster
+// way; then the rest, if few large jobs remain that fill the GPU by
+// themselves.  Jobs with an end criterion stay (it is decided in step).
+int split_jobs(std::vector<fdtd_engine_s*>& batched, std::vector<fdtd_engine_s*>& resident,
+               std::vector<fdtd_engine_s*>& own, int XC) {
+    std::vector<fdtd_engine_s*> fit, rest;
+    double sum = 0.0;
+    for (fdtd_engine_s* e : batched) {
+        if (e->E.idx16 && e->H.idx16 && e->end_crit == 0.0)
+            if (int rc = setup_resident(e)) return rc;
+        (e->res_ready && e->end_crit == 0.0 ? fit : rest).push_back(e);
+        if (fit.size() && fit.back() == e) sum += resident_us(e);
+    }
+    const bool all = sum <= batched_us(fit, XC);
+    for (fdtd_engine_s* e : fit) (all || resident_us(e) < nodes_of(e) / 58e3 ? resident : rest).push_back(e);
+    double alone = 0.0;
+    bool may = true;
+    for (const fdtd_engine_s* e : rest) {
+        alone += own_us(e);
+        may = may && e->end_crit == 0.0 && e->use_graphs;
+    }
+    if (may && alone < batched_us(rest, XC)) own.swap(rest);
+    batched.swap(rest);
+    return FDTD_OK;
+}
+
 // Why an engine cannot join a batch (0 = it can; the message is set).
 int batch_refusal(const fdtd_engine_s* e) {
     if (!e->use_tma || e->fused) {
@@ -240,7 +291,11 @@ using namespace wipems;
 struct fdtd_batch_s {
     int device = 0;
     cudaStream_t stream = nullptr;
-    std::vector<fdtd_engine_s*> jobs;
+    // the batched kernels' jobs, then the resident ones, then those on their
+    // own half-step kernels and streams (split_jobs)
+    std::vector<fdtd_engine_s*> jobs, own;
+    size_t first_resident = 0, first_own = 0;
+    cudaEvent_t ev_alone = nullptr, ev_jobs = nullptr;
     std::vector<Group> groups;
     DevBuf<BatchJob> d_jobs;
     DevBuf<TmaMaps> d_maps;
@@ -264,7 +319,6 @@ struct fdtd_batch_s {
     uint32_t graph_steps = 8;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t ev_jobs = nullptr;     // orders a run after the jobs' own streams
     double last_ms = 0;
     uint64_t last_launches = 0;
     uint64_t device_bytes = 0;
@@ -273,6 +327,7 @@ struct fdtd_batch_s {
         if (graph) cudaGraphExecDestroy(graph);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
+        if (ev_alone) cudaEventDestroy(ev_alone);
         if (ev_jobs) cudaEventDestroy(ev_jobs);
         for (cudaEvent_t e : ev_fork) cudaEventDestroy(e);
         for (cudaEvent_t e : ev_join) cudaEventDestroy(e);
@@ -392,7 +447,6 @@ int build_batch(const fdtd_engine_t* engines, uint32_t n, const fdtd_batch_opts*
     CK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&b->ev0));
     CK(cudaEventCreate(&b->ev1));
-    CK(cudaEventCreateWithFlags(&b->ev_jobs, cudaEventDisableTiming));
     int rc;
     for (uint32_t j = 0; j < n; ++j) {
         fdtd_engine_s* e = engines[j];
@@ -413,15 +467,18 @@ int build_batch(const fdtd_engine_t* engines, uint32_t n, const fdtd_batch_opts*
         if ((rc = engine_start(e))) return rc;
         CK(cudaStreamSynchronize(e->stream));
     }
+    std::vector<fdtd_engine_s*> batched(engines, engines + n), resident;
+    // (L2 bins are a schedule of the batched kernels: asked for, all jobs keep it)
+    if (!b->bin_bytes && (rc = split_jobs(batched, resident, b->own, b->XC))) return rc;
     // L2 bins: first fit by decreasing footprint (one bin when binning is off)
     std::vector<std::vector<fdtd_engine_s*>> binned;
     {
-        std::vector<fdtd_engine_s*> byfoot(engines, engines + n);
+        std::vector<fdtd_engine_s*> byfoot(batched);
         std::vector<uint64_t> load;
         if (b->bin_bytes)
             std::stable_sort(byfoot.begin(), byfoot.end(),
                              [](const fdtd_engine_s* a, const fdtd_engine_s* c) { return a->device_bytes > c->device_bytes; });
-        else
+        else if (!batched.empty())
             binned.emplace_back();
         for (fdtd_engine_s* e : byfoot) {
             if (!b->bin_bytes) {
@@ -495,6 +552,14 @@ int build_batch(const fdtd_engine_t* engines, uint32_t n, const fdtd_batch_opts*
         max_groups = std::max(max_groups, B.groups.size());
         b->bins.push_back(std::move(B));
     }
+    b->first_resident = b->jobs.size();
+    b->jobs.insert(b->jobs.end(), resident.begin(), resident.end());
+    b->first_own = b->jobs.size();
+    b->jobs.insert(b->jobs.end(), b->own.begin(), b->own.end());
+    b->total_nodes = 0;
+    for (const fdtd_engine_s* e : b->jobs) b->total_nodes += (uint64_t)e->N[0] * e->N[1] * e->N[2];
+    CK(cudaEventCreateWithFlags(&b->ev_alone, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&b->ev_jobs, cudaEventDisableTiming));
     if (b->chains > 1) {
         b->side.resize(max_groups, nullptr);
         b->ev_join.resize(max_groups, nullptr);
@@ -633,14 +698,39 @@ int fdtd_batch_iterate(fdtd_batch_t b, uint32_t n) {
     CK(cudaSetDevice(b->device));
     b->last_launches = 0;
     int rc;
-    if (b->graph_steps > 1 && n >= b->graph_steps && (rc = batch_graph(b))) return rc;
+    if (!b->bins.empty() && b->graph_steps > 1 && n >= b->graph_steps && (rc = batch_graph(b))) return rc;
     // what the jobs' own streams still hold (a reset, say) comes first
     for (fdtd_engine_s* e : b->jobs) {
         CK(cudaEventRecord(b->ev_jobs, e->stream));
         CK(cudaStreamWaitEvent(b->stream, b->ev_jobs, 0));
     }
     CK(cudaEventRecord(b->ev0, b->stream));
-    uint32_t left = n;
+    for (size_t j = b->first_resident; j < b->first_own; ++j) {
+        fdtd_engine_s* e = b->jobs[j];
+        e->last_launches = 0;
+        for (uint32_t left = n; left > 0;) {
+            const uint32_t run = resident_run(e, left);
+            if ((rc = launch_resident(e, run, b->stream))) return rc;
+            e->ts += run;
+            left -= run;
+        }
+        b->last_launches += e->last_launches;
+        CK(cudaMemcpyAsync(b->d_status.p + 4 * j, e->ctl.p, 4 * sizeof(int), cudaMemcpyDeviceToDevice, b->stream));
+    }
+    CK(cudaEventRecord(b->ev_alone, b->stream));
+    for (fdtd_engine_s* e : b->own) {
+        CK(cudaStreamWaitEvent(e->stream, b->ev_alone, 0));
+        const bool initial = e->need_initial_sample;  // a batch takes no sample before its first timestep
+        e->need_initial_sample = false;
+        rc = fdtd_engine_iterate_async(e, n);
+        e->need_initial_sample = initial;
+        if (rc) {
+            for (fdtd_engine_s* w : b->own) fdtd_engine_wait(w);
+            return rc;
+        }
+        b->last_launches += e->last_launches;
+    }
+    uint32_t left = b->bins.empty() ? 0 : n;
     while (left > 0) {
         if (b->graph && left >= b->graph_steps) {
             CK(cudaGraphLaunch(b->graph, b->stream));
@@ -653,16 +743,21 @@ int fdtd_batch_iterate(fdtd_batch_t b, uint32_t n) {
             if ((rc = bin_step(b, bi))) return rc;
         left -= 1;
     }
+    for (fdtd_engine_s* e : b->own) CK(cudaStreamWaitEvent(b->stream, e->ev1, 0));
     CK(cudaEventRecord(b->ev1, b->stream));
     CK(cudaEventSynchronize(b->ev1));
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
     b->last_ms = ms;
     // every job's control words in one copy: numTS, done, error word
-    const size_t nj = b->jobs.size();
+    const size_t nj = b->first_own;
     CK(cudaMemcpyAsync(b->h_status.data(), b->d_status.p, nj * 4 * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
     CK(cudaStreamSynchronize(b->stream));
     int first_rc = FDTD_OK;
+    for (fdtd_engine_s* e : b->own) {
+        rc = fdtd_engine_wait(e);
+        if (first_rc == FDTD_OK) first_rc = rc;
+    }
     for (size_t j = 0; j < nj; ++j) {
         fdtd_engine_s* e = b->jobs[j];
         const int* c = &b->h_status[4 * j];
@@ -677,7 +772,12 @@ int fdtd_batch_info(fdtd_batch_t b, fdtd_batch_stats* st) {
     if (!b || !st) return FDTD_ERR_ARG;
     std::memset(st, 0, sizeof(*st));
     st->num_jobs = (uint32_t)b->jobs.size();
-    st->num_groups = (uint32_t)b->groups.size();
+    std::set<std::array<int, 4>> alone;  // kernel variants of the jobs outside the batched kernels
+    for (size_t j = b->first_resident; j < b->jobs.size(); ++j) {
+        const fdtd_engine_s* e = b->jobs[j];
+        alone.insert({(int)e->E.idx16, (int)e->H.idx16, (int)e->geo_on, e->feat_e * 8 + e->feat_h});
+    }
+    st->num_groups = (uint32_t)(b->groups.size() + alone.size());
     st->num_bins = (uint32_t)b->bins.size();
     st->total_nodes = b->total_nodes;
     for (const Group& G : b->groups) {

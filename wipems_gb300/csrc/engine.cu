@@ -275,7 +275,10 @@ int start(fdtd_engine_s* e) {
     if (!e->started) {
         if ((rc = upload_probes(e))) return rc;
         e->started = true;
-        if (e->res_candidate && (rc = setup_resident(e))) return rc;
+        if (e->res_candidate) {
+            if ((rc = setup_resident(e))) return rc;
+            e->resident = e->res_ready;
+        }
         if (e->interval && e->use_graphs && !e->resident && (rc = build_chunk_graph(e))) return rc;
     }
     if (e->need_initial_sample) {
@@ -1029,7 +1032,7 @@ int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
     while (left > 0) {
         if (e->resident) {
             const uint32_t run = resident_run(e, left);
-            if ((rc = launch_resident(e, run))) return rc;
+            if ((rc = launch_resident(e, run, e->stream))) return rc;
             e->ts += run;
             left -= run;
             continue;

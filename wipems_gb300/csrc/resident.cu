@@ -49,7 +49,7 @@ Variant variant_of(int nodes, int feat, bool geo, bool late) {
     return {0, nullptr};
 }
 
-constexpr size_t kSampleBytes = (size_t)64 << 20;  // of a run's energy segments
+constexpr size_t kSampleBytes = (size_t)16 << 20;  // of a run's energy segments
 constexpr int kMaxRunSamples = 64;
 constexpr int kMaxRunFd = 256;
 constexpr uint32_t kMaxRun = 1024;  // timesteps of one launch
@@ -90,6 +90,7 @@ bool resident_plan(const int cov[3], const bool mur[3], int blocks, int nodes, i
 }
 
 int setup_resident(fdtd_engine_s* e) {
+    if (e->res_ready) return FDTD_OK;
     int sms = 0, coop = 0, smem = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->device));
@@ -148,7 +149,7 @@ int setup_resident(fdtd_engine_s* e) {
     a.fdval = e->res_fdval.p;
     a.eseg = e->energy_on_probe ? e->res_seg.p : nullptr;
     CK(cudaMemsetAsync(e->res_ll.p, 0, e->res_ll.n * sizeof(ulonglong2), e->stream));
-    e->resident = true;
+    e->res_ready = true;
     return FDTD_OK;
 }
 
@@ -160,21 +161,21 @@ uint32_t resident_run(const fdtd_engine_s* e, uint32_t n) {
     return n;
 }
 
-int launch_resident(fdtd_engine_s* e, uint32_t n) {
+int launch_resident(fdtd_engine_s* e, uint32_t n, cudaStream_t st) {
     ResArgs a = e->ra;
     a.ts0 = (int)e->ts;
     a.nsteps = (int)n;
     void* args[] = {&e->g, &a, &e->ps};
     CK(cudaLaunchCooperativeKernel(e->res_kernel, dim3((unsigned)(a.p[0] * a.p[1] * a.p[2])),
-                                   dim3((unsigned)e->res_threads), args, (size_t)e->res_smem, e->stream));
+                                   dim3((unsigned)e->res_threads), args, (size_t)e->res_smem, st));
     const int count = e->interval ? (int)((e->ts + n) / e->interval - e->ts / e->interval) : 0;
     const int first = e->interval ? (int)((e->ts / e->interval + 1) * e->interval) : 0;
     if (count && a.eseg) {
-        k_resident_planes<<<dim3(e->N[0] - 1, (unsigned)count), 256, 0, e->stream>>>(e->g, a.eseg, a.seg_stride,
+        k_resident_planes<<<dim3(e->N[0] - 1, (unsigned)count), 256, 0, st>>>(e->g, a.eseg, a.seg_stride,
                                                                                    e->res_plane.p);
         e->last_launches += 1;
     }
-    k_resident_samples<<<std::max(1, count), 256, 0, e->stream>>>(e->p_ts(), (int)n, count, first, (int)e->interval,
+    k_resident_samples<<<std::max(1, count), 256, 0, st>>>(e->p_ts(), (int)n, count, first, (int)e->interval,
                                                                 e->ps, e->g, a.pval, a.nentry, e->res_plane.p,
                                                                 a.eseg ? 1 : 0, e->ticket.p, kEps0, kMue0);
     e->last_launches += 2;
@@ -182,7 +183,7 @@ int launch_resident(fdtd_engine_s* e, uint32_t n) {
     if (fds) {
         ProbeSet ps = e->ps;
         ps.vals = a.fdval;
-        k_fd_accumulate<<<1, 256, std::max<size_t>(8, ps.nprobe * sizeof(double)), e->stream>>>(
+        k_fd_accumulate<<<1, 256, std::max<size_t>(8, ps.nprobe * sizeof(double)), st>>>(
             e->p_ts(), (int)(e->ts + n), ps, e->g, e->fd, ((int)e->ts / f + 1) * f, f, fds, a.nentry);
         e->last_launches += 1;
     }
