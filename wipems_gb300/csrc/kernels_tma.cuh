@@ -327,7 +327,11 @@ __device__ __forceinline__ bool volt_tile(const DevGrid& g, const TmaMaps& m, co
 }
 
 // ------------------------------------------------------------- H half-step
-// One tile of the current update (see volt_tile).  es/ec/hs/hc: the
+// One tile of the current update (see volt_tile), marching from the highest
+// plane of the chunk to the lowest: the x+1 voltages of a node are then its
+// own of the plane before, in registers, as the x-1 currents of the voltage
+// update are.  (Marching upwards read them from the next ring stage: a second
+// wait per plane and one more plane loaded per chunk.)  es/ec/hs/hc: the
 // thread's Kahan sums of V^2 and I^2, accumulated when energy is set.
 template <typename IdxT, int FEAT, bool GEO, int TY = TMA_TY>
 __device__ __forceinline__ bool curr_tile(const DevGrid& g, const TmaMaps& m, const TileInfo& ti, int bx, int by,
@@ -342,33 +346,27 @@ __device__ __forceinline__ bool curr_tile(const DevGrid& g, const TmaMaps& m, co
     const int z = z0 + tz, y = y0 + ty;
     const int x0 = bz * XC;
     const int x1 = min(x0 + XC, g.Nx - 1);
-    const int nplanes = x1 - x0;      // planes updated
-    const int nload = nplanes + 1;    // plane x1 is read as the x+1 neighbour
+    const int nplanes = x1 - x0;
     const bool active = (z < g.Nz - 1) && (y < g.Ny - 1);
     const long long C = g.comp;
     const int zl = min(z0 + 31, g.Nz - 1), yl = min(y0 + TY - 1, g.Ny - 1);
     const uint32_t base = ring;
 
-    auto issue = [&](int r, int s) {  // thread 0: plane x0+r into ring stage s
-        const int x = x0 + r;
+    auto issue = [&](int r, int s) {  // thread 0: plane x1-1-r into ring stage s
+        const int x = x1 - 1 - r;
         float* st = smem + (size_t)s * L::STAGE;
-        const bool upd = r < nplanes;  // plane x1 only contributes V
-        const bool up = UPML && upd && tile_has_upml(ti, x, y0, yl, z0, zl);
-        const uint32_t bytes =
-            L::HALO_BYTES + (upd ? L::OWN_BYTES + L::IDX_BYTES : 0) + (up ? L::OWN_BYTES : 0);
-        mbar_expect_tx(&bars[s], bytes);
+        const bool up = UPML && tile_has_upml(ti, x, y0, yl, z0, zl);
+        mbar_expect_tx(&bars[s], L::HALO_BYTES + L::OWN_BYTES + L::IDX_BYTES + (up ? L::OWN_BYTES : 0));
         tma_4d(st, &m.V_halo, &bars[s], z0, y0, x, 0);
-        if (upd) {
-            tma_4d(st + L::HALO_A, &m.I_own, &bars[s], z0, y0, x, 0);
-            tma_3d(st + L::HALO_A + L::OWN, &m.idxH, &bars[s], z0, y0, x);
-        }
+        tma_4d(st + L::HALO_A, &m.I_own, &bars[s], z0, y0, x, 0);
+        tma_3d(st + L::HALO_A + L::OWN, &m.idxH, &bars[s], z0, y0, x);
         if (up) tma_4d(st + L::OFF_FLUX, &m.FI_own, &bars[s], z0, y0, x, 0);
     };
 
     int issued = 0;
     if (nplanes > 0 && tid == 0) {
         fence_proxy_async();
-        for (RingPos ip(base, STAGES); issued < min(STAGES - 1, nload); ++issued, ip.next(STAGES))
+        for (RingPos ip(base, STAGES); issued < min(STAGES - 1, nplanes); ++issued, ip.next(STAGES))
             issue(issued, ip.s);
     }
     const long long yz = (long long)y * g.Nzp + z;
@@ -380,33 +378,33 @@ __device__ __forceinline__ bool curr_tile(const DevGrid& g, const TmaMaps& m, co
         gzE = __ldg(g.geo + 2 * S + g.Nx + g.Ny + z);
         gzI = __ldg(g.geo + 3 * S + g.Nx + g.Ny + z);
     }
-    float* Ip = g.I + (long long)x0 * g.sx + yz;
+    float n1 = 0.f, n2 = 0.f;  // V1, V2 at x+1
+    if (active && nplanes > 0) {
+        const long long o = (long long)x1 * g.sx + yz;
+        n1 = g.V[C + o];
+        n2 = g.V[2 * C + o];
+    }
+    float* Ip = g.I + (long long)(x1 - 1) * g.sx + yz;
     bool aborted = false;
     int r = 0;
     RingPos cp(base, STAGES);  // stage of plane r
-    for (; r < nplanes; ++r, Ip += g.sx, cp.next(STAGES)) {
-        if (tid == 0 && issued < nload && issued == r + STAGES - 1) {
+    for (; r < nplanes; ++r, Ip -= g.sx, cp.next(STAGES)) {
+        if (tid == 0 && issued < nplanes && issued == r + STAGES - 1) {
             // plane r + STAGES - 1 goes into the stage plane r - 1 freed
             fence_proxy_async();
             issue(issued, cp.s == 0 ? STAGES - 1 : cp.s - 1);
             ++issued;
         }
-        const int s = cp.s;
-        const int sn = s + 1 == STAGES ? 0 : s + 1;  // plane r + 1 (its V is the x+1 neighbour)
-        bool ok = mbar_wait(&bars[s], cp.ph);
-        ok = ok && mbar_wait(&bars[sn], cp.ph ^ (uint32_t)(sn == 0));
-        const int x = x0 + r;
+        const bool ok = mbar_wait(&bars[cp.s], cp.ph);
+        const int x = x1 - 1 - r;
         float ev[3] = {0.f, 0.f, 0.f}, eh[3] = {0.f, 0.f, 0.f};  // energy terms of this node
         if (ok && active) {
-            const float* st = smem + (size_t)s * L::STAGE;
-            const float* stn = smem + (size_t)sn * L::STAGE;
+            const float* st = smem + (size_t)cp.s * L::STAGE;
             const float* sV0 = st;
             const float* sV1 = st + (TY + 1) * HW;
             const float* sV2 = st + 2 * (TY + 1) * HW;
             const int hi = ty * HW + tz;
             const float c0 = sV0[hi], c1 = sV1[hi], c2 = sV2[hi];
-            const float n1 = stn[(TY + 1) * HW + hi];
-            const float n2 = stn[2 * (TY + 1) * HW + hi];
             float curl[3];
             curl[0] = __fadd_rn(__fsub_rn(__fsub_rn(c2, sV2[hi + HW]), c1), sV1[hi + 1]);
             curl[1] = __fadd_rn(__fsub_rn(__fsub_rn(c0, sV0[hi + 1]), c2), n2);
@@ -429,6 +427,8 @@ __device__ __forceinline__ bool curr_tile(const DevGrid& g, const TmaMaps& m, co
             Ip[0] = cu[0];
             Ip[C] = cu[1];
             Ip[2 * C] = cu[2];
+            n1 = c1;
+            n2 = c2;
             ev[0] = c0; ev[1] = c1; ev[2] = c2;
             eh[0] = cu[0]; eh[1] = cu[1]; eh[2] = cu[2];
         }
@@ -440,7 +440,7 @@ __device__ __forceinline__ bool curr_tile(const DevGrid& g, const TmaMaps& m, co
             break;
         }
     }
-    ring = base + (uint32_t)(nplanes > 0 ? nload : 0);
+    ring = base + (uint32_t)max(nplanes, 0);
     if (aborted && tid == 0) {
         atomicOr(ti.d_err, 4);
         for (int k = r; k < issued; ++k) {
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(TY * 32) k_curr_tma(const DevGrid g, const __g
     if (*g.d_done) return;
     init_ring(bars, STAGES);
     uint32_t ring = 0;
-    // x-chunks in descending order: blocks are dispatched roughly in
+    // x-chunks (and the planes in them) in descending order: blocks are dispatched roughly in
     // blockIdx order, and the voltage kernel before this one ended on the
     // highest chunks, whose voltages (just written) and currents (just read)
     // are still partly in L2.  The next voltage kernel, in ascending order,
