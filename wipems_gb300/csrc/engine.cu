@@ -580,7 +580,7 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
         // about 1280 resident threads per SM (5 blocks of 32 x 8, 10 of 32 x 4)
         e->XC = auto_x_chunk({e->N}, (uint64_t)(1280 / (32 * e->tma_ty)) * (uint64_t)sms, TMA_TY,
-                             e->use_tma && !e->fused);
+                             !e->use_tma || e->fused ? 16 : c->E.adex_orders || c->H.adex_orders ? 2 : 6);
     }
     e->comp = c->comp;
     e->geo_on = c->geo;

@@ -207,19 +207,21 @@ namespace wipems {
 // plane each), blocks run in waves of `resident`, so the step costs
 // ceil(blocks / resident) * (2 + x_chunk); a chunk that leaves SMs idle in the
 // only wave is skipped, ties go to the longer chunk (fewer halo-plane
-// re-reads).  lines: the jobs' (Nx, Ny, Nz) triples.  `single`: one job on
+// re-reads).  lines: the jobs' (Nx, Ny, Nz) triples.  longest <= 6: one job on
 // the half-step kernels, whose chunks are 1, 2 or 4 planes, or 6 with eight
 // waves to spare: longer ones end the voltage half-step far from where the
 // current one starts, and what it left in L2 is gone (257^3 UPML 16 planes
 // 266 us per step, 8: 261, 6: 256, 4: 260; 161^3 UPML 8: 88, 6: 83, 4: 81.6;
-// 257^3 PEC 16: 202, 6 and 4: 194).  Otherwise 1, 2, 4, 8 or 16.
+// 257^3 PEC 16: 202, 6 and 4: 194).  Otherwise 1, 2, 4, 8 or 16.  With
+// dispersion orders above 1 at most 2: the blocks inside such materials take
+// several times as long as the others (106 x 101 x 96 lines 4 planes 35.0 us
+// per step, 2: 31.5).
 inline int auto_x_chunk(const std::vector<const uint32_t*>& lines, uint64_t resident, int ty = TMA_TY,
-                        bool single = false) {
+                        int longest = 16) {
     int best = 1;
     uint64_t best_cost = ~0ull;
-    static const int own[] = {6, 4, 2, 1}, shared[] = {16, 8, 4, 2, 1};
-    for (int k = 0; k < (single ? 4 : 5); ++k) {
-        const int xc = single ? own[k] : shared[k];
+    for (int xc : {16, 8, 6, 4, 2, 1}) {
+        if (xc > longest || (xc == 6 && longest != 6)) continue;
         uint64_t items = 0;
         for (const uint32_t* N : lines)
             items += (uint64_t)((N[2] - 1 + 31) / 32) * ((N[1] - 1 + ty - 1) / ty) * ((N[0] - 1 + xc - 1) / xc);

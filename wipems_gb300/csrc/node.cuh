@@ -234,14 +234,15 @@ __device__ __forceinline__ void update_node(const DevGrid& g, float fld[3], cons
             }
         }
     }
-    // dispersion orders 1..3 (materials with several poles): the same update
-    // of each order's states from the same old field, in order
+    // dispersion orders 1..3 (materials with several poles): the update of
+    // each order's states from the same old field, in order
     // (engine_ext_lorentzmaterial.cpp:80-121 loop over o); the new states
-    // stay in global memory and are subtracted after the node update
+    // wait in registers for the subtraction after the node update
+    float adex[kExtraOrders][3];
     if ((FEAT & FEAT_ADEX) && (flags & TF_ADEX_ALL)) {
         float* Ax = H ? g.AIx : g.AVx;
         float* Lx = H ? g.LIx : g.LVx;
-#pragma unroll 1
+#pragma unroll
         for (int k = 0; k < kExtraOrders; ++k) {
             if (!(flags & (TF_ADEX << k))) continue;
             const float4* ta = T.adex + ((long long)k * T.ntup + t) * TAB_ADE;
@@ -266,6 +267,7 @@ __device__ __forceinline__ void update_node(const DevGrid& g, float fld[3], cons
                 a = __fmul_rn(a, kint[n]);
                 a = __fadd_rn(a, __fmul_rn(kext[n], f));
                 As[n * C + o] = a;
+                adex[k][n] = a;
             }
         }
     }
@@ -294,12 +296,11 @@ __device__ __forceinline__ void update_node(const DevGrid& g, float fld[3], cons
     }
     // V -= ADE of each further order, order by order (engine_ext_dispersive.cpp:76-132)
     if ((FEAT & FEAT_ADEX) && (flags & TF_ADEX_ALL)) {
-        const float* Ax = H ? g.AIx : g.AVx;
-#pragma unroll 1
+#pragma unroll
         for (int k = 0; k < kExtraOrders; ++k) {
             if (!(flags & (TF_ADEX << k))) continue;
 #pragma unroll
-            for (int n = 0; n < 3; ++n) fld[n] = __fsub_rn(fld[n], Ax[(long long)k * 3 * C + n * C + o]);
+            for (int n = 0; n < 3; ++n) fld[n] = __fsub_rn(fld[n], adex[k][n]);
         }
     }
     if (flags & TF_EXC) excite_node<H>(g, fld, t, numTS);
