@@ -136,14 +136,23 @@ int setup_resident(fdtd_engine_s* e) {
     a.d_err = e->p_err();
     a.seg_stride = (long long)(e->N[0] - 1) * (e->N[1] - 1) * e->g.nzt;
     e->res_samples = (int)std::max<size_t>(1, std::min<size_t>(kMaxRunSamples, kSampleBytes / (8 * a.seg_stride)));
-    int rc;
     uint64_t& tot = e->device_bytes;
-    if ((rc = e->res_ll.alloc(std::max<long long>(1, 4 * a.ll_pairs), tot, e->stream)) ||
-        (rc = e->res_pval.alloc(std::max<size_t>(1, entries * e->res_samples), tot, e->stream)) ||
-        (fd && (rc = e->res_fdval.alloc(std::max<size_t>(1, entries * kMaxRunFd), tot, e->stream))) ||
-        (rc = e->res_seg.alloc(a.seg_stride * e->res_samples, tot, e->stream)) ||
-        (rc = e->res_plane.alloc((size_t)(e->N[0] - 1) * e->res_samples, tot, e->stream)))
-        return rc;
+    const uint64_t before = tot;
+    if (e->res_ll.alloc(std::max<long long>(1, 4 * a.ll_pairs), tot, e->stream) ||
+        e->res_pval.alloc(std::max<size_t>(1, entries * e->res_samples), tot, e->stream) ||
+        (fd && e->res_fdval.alloc(std::max<size_t>(1, entries * kMaxRunFd), tot, e->stream)) ||
+        e->res_seg.alloc(a.seg_stride * e->res_samples, tot, e->stream) ||
+        e->res_plane.alloc((size_t)(e->N[0] - 1) * e->res_samples, tot, e->stream)) {
+        // no memory left for it: the half-step kernels need none
+        cudaGetLastError();
+        e->res_ll.release();
+        e->res_pval.release();
+        e->res_fdval.release();
+        e->res_seg.release();
+        e->res_plane.release();
+        tot = before;
+        return FDTD_OK;
+    }
     a.ll = e->res_ll.p;
     a.pval = e->res_pval.p;
     a.fdval = e->res_fdval.p;
