@@ -39,15 +39,18 @@ def tune(cop, stages=DEFAULT_STAGES, xchunks=DEFAULT_XCHUNK, steps: int = 30, de
     """Times every (kernel, tile_y, stages, x_chunk) combination the way the
     engine runs -- CUDA-graph chunks of one probe interval, device time from
     CUDA events over `steps` timesteps -- and returns (best, table), best
-    minimising the time per timestep.  kernels may add "fused" (the
-    single-pass kernel, where the grid allows it; its tile is fixed)."""
+    minimising the time per timestep.  The engine's own choice (kernel "auto"
+    with no tiling given: resident timesteps where the grid fits) is always a
+    candidate.  kernels may add "fused" (the single-pass kernel, where the
+    grid allows it; its tile is fixed)."""
     from ._abi import FdtdError
     from .fdtd import Engine
     table = []
-    for k in kernels:
+    for k in ("auto", *kernels):
+        own = k == "auto"
         for ty in (tile_ys if k == "tma" else (0,)):
-            for s in stages:
-                for xc in xchunks:
+            for s in (0,) if own else stages:
+                for xc in (0,) if own else xchunks:
                     try:
                         eng = Engine(cop, device=device, stages=s, x_chunk=xc, max_timesteps=2 * steps + 64,
                                      kernel=k, tile_y=ty)
@@ -57,7 +60,7 @@ def tune(cop, stages=DEFAULT_STAGES, xchunks=DEFAULT_XCHUNK, steps: int = 30, de
                     eng.reset()
                     eng.iterate(steps)
                     ms, _ = eng.last_timing()
-                    tile = eng.stats()["tile_y"]
+                    tile = 0 if own else eng.stats()["tile_y"]
                     eng.close()
                     table.append(dict(kernel=k, tile_y=tile, stages=s, x_chunk=xc, ms_step=ms / steps))
                     if verbose:

@@ -1202,12 +1202,13 @@ int grow_dump(fdtd_engine_s* e, size_t floats) {
 // a share per thread.  A fresh array's pages do not exist yet, and faulting
 // them in one by one under the copy takes many times the copy: both fields of
 // 257^3 lines (408 MB) took 335 ms to read, 6.4 ms with their pages mapped by
-// 16 threads first.  Below 4 MB the copy alone is a fraction of a millisecond.
+// 16 threads first.  Small arrays (over the allocator's usual threshold for
+// fresh pages) are touched by the calling thread alone.
 void touch_pages(void* p, size_t bytes) {
-    if (bytes < (size_t)4 << 20) return;
+    if (bytes < (size_t)256 << 10) return;
     const size_t page = 4096;
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned nt = (unsigned)std::min<size_t>(std::min(hw, 16u), bytes >> 21);
+    const unsigned nt = (unsigned)std::max<size_t>(1, std::min<size_t>(std::min(hw, 16u), bytes >> 21));
     auto part = [=](unsigned k) {
         volatile char* b = static_cast<volatile char*>(p);
         const size_t lo = bytes / nt * k, hi = k + 1 == nt ? bytes : bytes / nt * (k + 1);
