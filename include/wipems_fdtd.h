@@ -438,9 +438,13 @@ typedef struct {
     int      energy_on_probe; /* fuse the energy reduction into sample steps */
     int      tile_y;          /* kernel tile rows (0 = autotuned default) */
     int      x_chunk;         /* x planes per block (0 = chosen from the grid
-                                 size by a wave model: 1, 2, 4, 8 or 16) */
-    int      kernel;          /* 0 = default: the TMA-pipelined two-pass
-                                     kernels (3),
+                                 size by a wave model) */
+    int      kernel;          /* 0 = default: with no tiling given (tile_y,
+                                     x_chunk, stages 0) and no end criterion,
+                                     a grid that fits in the GPU's shared
+                                     memory runs resident; otherwise the
+                                     TMA-pipelined two-pass kernels (3).
+                                     Either way the same bits,
                                  1 = direct-load kernels,
                                  2 = fused single-pass TMA kernel (E and H of
                                      a timestep in one x-march, double-
@@ -655,6 +659,10 @@ typedef struct {
     uint32_t x_chunk;   /* x planes per work item in use */
 } fdtd_batch_stats;
 
+/* Jobs without an end criterion that run faster resident (see
+ * fdtd_engine_opts.kernel), or alone when few large ones remain, are stepped
+ * that way instead of by the batched kernels (not with bin_mib); num_groups
+ * counts their kernel variants too. */
 int fdtd_batch_create(const fdtd_engine_t* engines, uint32_t n,
                       const fdtd_batch_opts* opts, fdtd_batch_t* out);
 /* *ok = 1 when fdtd_batch_create would take the engine (two-pass TMA

@@ -81,7 +81,7 @@ struct DevGrid {
     // energy on sample steps, in an order fixed by the grid alone: one
     // (sum V^2, sum I^2) float pair per segment (x < Nx-1, y < Ny-1, 32-node
     // z tile zt < nzt) written by the warp that updates it, then one double
-    // pair per x plane (k_energy_planes), summed in x order by the sampler
+    // pair per x plane, summed by the sampler in a fixed order (total_energy)
     float2* eseg;        // [(Nx-1)*(Ny-1)*nzt]
     double2* eplane;     // [Nx-1]
     int nzt;             // ceil((Nz-1)/32)
