@@ -118,9 +118,11 @@ int check_launch() {
     return FDTD_OK;
 }
 
-void launch_mur(fdtd_engine_s* e, int ts_off, int stage) {
-    const unsigned blocks = std::min<unsigned>((e->mur.total + 255) / 256, 1024u);
-    k_mur<<<blocks, 256, 0, e->stream>>>(e->g, e->mur, ts_off, stage);
+void launch_mur(fdtd_engine_s* e, int ts_off, int stage, bool next = false) {
+    RlcSet rs = e->rlc;
+    if (stage != 1 || !e->mur_rlc) rs.count = 0;
+    const unsigned blocks = std::min<unsigned>((e->mur.total + rs.count + 255) / 256, 1024u);
+    k_mur<<<blocks, 256, 0, e->stream>>>(e->g, e->mur, rs, ts_off, stage, next ? 1 : 0);
     e->last_launches += 1;
 }
 
@@ -132,18 +134,19 @@ void launch_rlc(fdtd_engine_s* e, int ts_off) {
 
 // The voltage half-step with the passes that surround it: Mur pre-update,
 // the voltage kernel, Mur post-update, lumped RLC, Mur apply (the
-// reference's hook order for these extensions).
-void launch_volt_hooks(fdtd_engine_s* e, int ts_off) {
-    if (e->mur.nface) launch_mur(e, ts_off, 0);
+// reference's hook order for these extensions).  first: the run's first
+// timestep; last: its last one (no pre-update of the next).
+void launch_volt_hooks(fdtd_engine_s* e, int ts_off, bool first, bool last) {
+    if (e->mur.nface && first) launch_mur(e, ts_off, 0);
     launch_volt(e, ts_off);
     if (e->mur.nface) launch_mur(e, ts_off, 1);
-    if (e->rlc.count) launch_rlc(e, ts_off);
-    if (e->mur.nface) launch_mur(e, ts_off, 2);
+    if (e->rlc.count && !e->mur_rlc) launch_rlc(e, ts_off);
+    if (e->mur.nface) launch_mur(e, ts_off, 2, !last);
 }
 
-int launch_step(fdtd_engine_s* e, int ts_off, bool energy) {
+int launch_step(fdtd_engine_s* e, int ts_off, bool energy, bool last) {
     if (e->mur.nface || e->rlc.count) {
-        launch_volt_hooks(e, ts_off);
+        launch_volt_hooks(e, ts_off, ts_off == 0, last);
         launch_curr(e, ts_off, energy);
         e->last_launches += 2;
         return check_launch();
@@ -163,7 +166,7 @@ int launch_step(fdtd_engine_s* e, int ts_off, bool energy) {
 // after them); energy: the last one writes the energy segments
 int launch_steps(fdtd_engine_s* e, uint32_t n, bool energy) {
     int rc = FDTD_OK;
-    for (uint32_t k = 0; k < n && rc == FDTD_OK; ++k) rc = launch_step(e, (int)k, energy && k + 1 == n);
+    for (uint32_t k = 0; k < n && rc == FDTD_OK; ++k) rc = launch_step(e, (int)k, energy && k + 1 == n, k + 1 == n);
     return rc;
 }
 
@@ -650,7 +653,8 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
         }
         size_t tot_n = 0;
         for (const MurFace& M : c->mur) tot_n += (size_t)M.n[0] * M.n[1];
-        if ((rc = e->mur_coef.alloc(2 * tot_n, tot, e->stream)) || (rc = e->mur_buf.alloc(2 * tot_n, tot, e->stream)))
+        if ((rc = e->mur_coef.alloc(2 * tot_n, tot, e->stream)) || (rc = e->mur_buf.alloc(2 * tot_n, tot, e->stream)) ||
+            (rc = e->mur_buf2.alloc(2 * tot_n, tot, e->stream)))
             return rc;
         CK(cudaMemsetAsync(e->mur_buf.p, 0, 2 * tot_n * sizeof(float), e->stream));
         std::vector<float> hc(2 * tot_n);
@@ -669,13 +673,33 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
             F.start_ts = (int)M.start_ts;
             F.cp = e->mur_coef.p + 2 * off;
             F.cpp = e->mur_coef.p + 2 * off + n;
-            F.bp = e->mur_buf.p + 2 * off;
-            F.bpp = e->mur_buf.p + 2 * off + n;
+            F.b[0] = e->mur_buf.p + 2 * off;
+            F.b[1] = e->mur_buf2.p + 2 * off;
             F.offset = (uint32_t)off;
             off += n;
         }
         e->mur.total = (uint32_t)tot_n;
         e->mur.idx16 = c->E.idx16 ? 1 : 0;
+        e->mur.exc = 0;
+        for (const MurFace& M : c->mur) {
+            const int nP = (M.ny + 1) % 3, nPP = (M.ny + 2) % 3;
+            for (uint32_t i = 0; i < M.n[0] && !e->mur.exc; ++i)
+                for (uint32_t j = 0; j < M.n[1]; ++j) {
+                    uint32_t p[3];
+                    p[M.ny] = M.line;
+                    p[nP] = i;
+                    p[nPP] = j;
+                    const size_t o = ((size_t)p[0] * e->N[1] + p[1]) * (size_t)e->Nzp + p[2];
+                    const uint32_t t = c->E.idx16 ? reinterpret_cast<const uint16_t*>(c->E.idx)[o]
+                                                  : reinterpret_cast<const uint32_t*>(c->E.idx)[o];
+                    uint32_t f;
+                    std::memcpy(&f, &c->E.main[(size_t)t * TAB_MAIN * 4 + 6], 4);
+                    if (f & TF_EXC) {
+                        e->mur.exc = 1;
+                        break;
+                    }
+                }
+        }
         for (int a = 0; a < 3; ++a) e->mur.trim[a] = c->trim_e[a] ? 1 : 0;
         CK(cudaMemcpyAsync(e->mur_coef.p, hc.data(), hc.size() * sizeof(float), cudaMemcpyHostToDevice, e->stream));
     }
@@ -701,6 +725,14 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
         CK(cudaMemsetAsync(e->rlc_state.p, 0, 7 * n * sizeof(float), e->stream));
         CK(cudaStreamSynchronize(e->stream));  // the host staging vectors end here
         e->rlc.count = (uint32_t)n;
+        // with Mur faces the edges run beside their post-update, unless one
+        // lies on a line that a face reads or writes
+        e->mur_rlc = e->mur.nface > 0;
+        for (size_t k = 0; k < n; ++k)
+            for (int f = 0; f < e->mur.nface; ++f) {
+                const uint32_t p = r.pos[e->mur.f[f].ny][k];
+                if ((int)p == e->mur.f[f].line || (int)p == e->mur.f[f].shift) e->mur_rlc = false;
+            }
         e->rlc.off = e->rlc_off.p;
         e->rlc.coef = e->rlc_coef.p;
         e->rlc.state = e->rlc_state.p;
@@ -1582,7 +1614,7 @@ int fdtd_engine_profile_kernels(fdtd_engine_t e, uint32_t n_steps, double* ms_vo
             launch_fused(e, 0, sample && e->energy_on_probe);
             CK(cudaEventRecord(ev[3 * k + 1], e->stream));
         } else {
-            launch_volt_hooks(e, 0);
+            launch_volt_hooks(e, 0, true, true);
             CK(cudaEventRecord(ev[3 * k + 1], e->stream));
             launch_curr(e, 0, sample && e->energy_on_probe);
         }

@@ -135,8 +135,9 @@ struct fdtd_engine_s {
     DevBuf<int> d_fd_dual, d_fd_count;
     FdSet fd{};
     // Mur ABC faces
-    DevBuf<float> mur_coef, mur_buf;
+    DevBuf<float> mur_coef, mur_buf, mur_buf2;
     MurSet mur{};
+    bool mur_rlc = false;  // the lumped RLC edges run in the Mur post-update's launch
     // lumped RLC edges
     DevBuf<float> rlc_coef, rlc_state;
     DevBuf<long long> rlc_off;

@@ -237,7 +237,7 @@ struct ResMur {
                 const int loc = (i + lP) * F.n1 + j + lQ;
                 node[count + q] = make_uint2(ol | os << 13 | (uint32_t)ny << 26 | (uint32_t)fi << 28 | (inert ? 1u << 31 : 0u),
                                              m1 | m2 << 6 | (exc ? 1u << 12 : 0u) | t << 16);
-                val[count + q] = make_float4(F.cp[loc], F.cpp[loc], F.bp[loc], F.bpp[loc]);
+                val[count + q] = make_float4(F.cp[loc], F.cpp[loc], 0.f, 0.f);
             }
             count += nP * nQ;
         }
@@ -290,24 +290,6 @@ struct ResMur {
             }
             if (!(e.y & act & 63u)) sV[comp(ny + 1) + ol] = v1;
             if (!(e.y >> 6 & act & 63u)) sV[comp(ny + 2) + ol] = v2;
-        }
-    }
-    // the values back to the engine's buffers
-    __device__ __forceinline__ void store(const MurSet& ms, int lx, int ly, int lz, int bx, int by, int bz) const {
-        int first = 0;
-        for (int fi = 0; fi < ms.nface; ++fi) {
-            const MurDev F = ms.f[fi];
-            const int ny = F.ny;
-            const int l0 = ny == 0 ? lx : ny == 1 ? ly : lz, n0 = ny == 0 ? bx : ny == 1 ? by : bz;
-            const int lP = ny == 0 ? ly : ny == 1 ? lz : lx, nP = ny == 0 ? by : ny == 1 ? bz : bx;
-            const int lQ = ny == 0 ? lz : ny == 1 ? lx : ly, nQ = ny == 0 ? bz : ny == 1 ? bx : by;
-            if (F.line < l0 || F.line >= l0 + n0) continue;
-            for (int q = threadIdx.x; q < nP * nQ; q += blockDim.x) {
-                const int i = q / nQ, j = q - i * nQ, loc = (i + lP) * F.n1 + j + lQ;
-                F.bp[loc] = val[first + q].z;
-                F.bpp[loc] = val[first + q].w;
-            }
-            first += nP * nQ;
         }
     }
 };
@@ -626,7 +608,6 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
         }
     }
     if (!ok) atomicOr(a.d_err, 4);
-    if (LATE && late) mur.store(a.mur, lx, ly, lz, bx, by, bz);
     for (int r = warp; r < rows; r += nwarps) {
         const int x = r / by, y = r - x * by;
         const long long go = g0 + (long long)x * g.sx + (long long)y * g.Nzp;
