@@ -53,7 +53,8 @@ _MIX = [BC_MUR, BC_MUR, BC_PEC, BC_MUR, BC_MUR, BC_PMC]
     ((33, 34, 35), BC_MUR, False, ()), ((22, 31, 65), _MIX, False, ("rlc",)), ((40, 25, 33), BC_MUR, True, ("rlc",)),
     ((21, 22, 40), BC_PML, False, ("rlc",)), ((30, 26, 37), BC_MUR, False, ("drude",)),
     ((30, 27, 64), _MIX, False, ("drude", "lorentz")), ((29, 28, 36), BC_PML, False, ("drude", "lorentz")),
-    ((28, 30, 33), BC_PEC, False, ("lorentz", "rlc"))])
+    ((28, 30, 33), BC_PEC, False, ("lorentz", "rlc")), ((30, 31, 38), BC_PML, True, ("drude", "lorentz")),
+    ((33, 26, 35), BC_MUR, True, ("drude",)), ((27, 31, 36), BC_PEC, True, ("lorentz",))])
 def test_resident_equals_direct(n, wall, graded, media):
     cop = CompressedOperator(_op(n, wall, graded, media))
     a, b = Engine(cop, max_timesteps=300), Engine(cop, max_timesteps=300, kernel="direct")
