@@ -1,0 +1,73 @@
+"""Resident runs (the default kernel choice) against the kernels that read the
+fields of every timestep from memory: the same bits."""
+import numpy as np
+import pytest
+
+from wipems_gb300 import CompressedOperator, Engine, Operator, Scene
+from wipems_gb300.fdtd import BC_PEC, BC_PMC, BC_PML
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("libs")]
+
+
+def _scene(n, wall=BC_PEC):
+    s = Scene(*[np.arange(k, dtype=float) for k in n], 1e-3)
+    s.set_boundary([wall] * 6, [4 if wall == BC_PML else 0] * 6)
+    s.set_gauss_excite(20e9, 20e9, 300)
+    c = [k // 2 for k in n]
+    s.add_excitation(c, [c[0], c[1], c[2] + 1], [0.3, 0.0, 1.0])
+    s.add_probe([c[0], c[1], 0], [c[0], c[1], n[2] - 1], 0)
+    return s
+
+
+def _same(a, b):
+    sa, sb = a.samples(), b.samples()
+    for x, y in zip([*a.fields(), sa.ts, sa.values, sa.energy], [*b.fields(), sb.ts, sb.values, sb.energy]):
+        assert x.tobytes() == y.tobytes()
+
+
+@pytest.mark.parametrize("n,wall", [((21, 21, 21), BC_PEC), ((22, 35, 40), BC_PEC), ((24, 25, 33), BC_PML),
+                                    ((23, 20, 26), BC_PMC)])
+def test_probes_on_last_lines(n, wall):
+    """Probes that read the last line of every axis, which the voltage update
+    leaves out at a PEC or UPML wall: current loops around whole
+    cross-sections, field probes and voltage lines on it, and what the caller
+    wrote there."""
+    s = _scene(n, wall)
+    top = [k - 1 for k in n]
+    for a in range(3):
+        lo, hi = [0, 0, 0], list(top)
+        lo[a] = hi[a] = n[a] // 3
+        s.add_probe(lo, hi, 1, norm_dir=a)
+        at = [k // 2 for k in n]
+        at[a] = top[a]
+        s.add_probe(at, at, 2)
+        s.add_probe(at, at, 3)
+        line = list(top)
+        line[a] = 0
+        s.add_probe(line, top, 0)
+    s.add_probe(top, top, 2)
+    cop = CompressedOperator(Operator(s))
+    assert any(p.enabled and max(p.stop[a] == top[a] for a in range(3)) for p in cop.op.probes if p.type == 1)
+    es = [Engine(cop, max_timesteps=300, kernel=k) for k in ("auto", "tma")]
+    for e in es:
+        e.set_frequencies(np.linspace(5e9, 30e9, 3), fd_interval=5)
+        e.iterate(20)
+        for a in range(3):  # nodes of the probes: on the loops, at the field probe, on the voltage line
+            b = (a + 1) % 3
+            at = list(top)
+            at[a], at[b] = n[a] // 3, n[b] // 2
+            e.set_curr(b, *at, 0.125 + a)
+            at = [k // 2 for k in n]
+            at[a] = top[a]
+            e.set_volt(a, *at, -0.5 - a)
+            at = list(top)
+            at[a] = 3
+            e.set_volt(a, *at, 2.0 + a)
+        e.iterate(61)
+        e.iterate(30)
+    _same(*es)
+    assert es[0].fd_results()[0].tobytes() == es[1].fd_results()[0].tobytes()
+    s = es[1].samples()
+    assert np.count_nonzero(np.abs(s.values[s.ts > 25]).max(axis=0) > 0.1) >= 6  # the written values are seen
+    for e in es:
+        e.close()

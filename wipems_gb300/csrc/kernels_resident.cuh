@@ -65,7 +65,7 @@ constexpr uint32_t RT_ROW = 16u << 16;  // this half-step updates the row
 constexpr uint32_t RT_Z = 32u << 16;    // E: node z-1 of lane 0 is in the box
 
 struct ResArgs {
-    int cov[3];              // nodes the boxes cover (lines that never change are left out)
+    int cov[3];              // nodes the boxes cover (lines that no timestep changes are left out)
     int p[3];                // boxes per axis
     int ne[3];               // extent of the voltage update
     int ts0, nsteps;         // numTS at the start, timesteps of this run
@@ -391,6 +391,18 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
         const int X = (int)(pe.off / g.sx);
         const int rem = (int)(pe.off - (long long)X * g.sx);
         const int Y = rem / g.Nzp, Z = rem - Y * g.Nzp;
+        if (X >= a.cov[0] || Y >= a.cov[1] || Z >= a.cov[2]) {
+            // on a line that no box covers: no timestep changes it, so the
+            // first block writes its value for every sample of the run
+            if (blockIdx.x == 0) {
+                const float v = (pe.field ? g.I : g.V)[pe.comp * C + pe.off];
+                const int ns = a.interval > 0 ? (a.ts0 + a.nsteps) / a.interval - a.ts0 / a.interval : 0;
+                const int nf = a.fd_interval > 0 ? (a.ts0 + a.nsteps) / a.fd_interval - a.ts0 / a.fd_interval : 0;
+                for (int m = 0; m < ns; ++m) a.pval[(long long)m * a.nentry + k] = v;
+                for (int m = 0; m < nf; ++m) a.fdval[(long long)m * a.nentry + k] = v;
+            }
+            continue;
+        }
         const int x = X - lx, y = Y - ly, z = Z - lz;
         if (x < 0 || x >= bx || y < 0 || y >= by || z < 0 || z >= bz) continue;
         ent[atomicAdd(&s_nent, 1)] =
