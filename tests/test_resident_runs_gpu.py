@@ -71,3 +71,20 @@ def test_probes_on_last_lines(n, wall):
     assert np.count_nonzero(np.abs(s.values[s.ts > 25]).max(axis=0) > 0.1) >= 6  # the written values are seen
     for e in es:
         e.close()
+
+
+@pytest.mark.parametrize("nprobe,interval", [(1, 3), (11, 1), (40, 4)])
+def test_samples_without_energies(nprobe, interval):
+    """Many samples per run and no energy sums (whose barriers would also
+    order the sample rows)."""
+    s = _scene((22, 25, 30))
+    for k in range(nprobe - 1):
+        s.add_probe([k % 21, 12, 0], [k % 21, 12, 29 - k % 5], 0, weight=1.0 + k)
+    cop = CompressedOperator(Operator(s))
+    es = [Engine(cop, max_timesteps=400, probe_interval=interval, energy_on_probe=False, kernel=k)
+          for k in ("auto", "tma")]
+    for e in es:
+        e.iterate(7)
+        e.iterate(200)
+    _same(*es)
+    assert es[0].samples().values.shape == (207 // interval + 1, nprobe)

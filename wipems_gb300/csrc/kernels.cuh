@@ -427,10 +427,12 @@ static __global__ void __launch_bounds__(256) k_energy_planes(const DevGrid g) {
 }
 
 // True in every thread of the block that arrives last of `blocks` (its
-// reads then see what the others wrote before); the ticket is back at zero
-// for the next launch.
+// reads then see what the others wrote before, and the others have read what
+// it will write: a block arrives once all of its threads have come here);
+// the ticket is back at zero for the next launch.
 __device__ __forceinline__ bool last_block(unsigned* ticket, unsigned blocks) {
     __shared__ int s_last;
+    __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         s_last = atomicInc(ticket, blocks - 1) == blocks - 1;
