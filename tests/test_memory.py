@@ -1,0 +1,21 @@
+"""Host-side memory handling of the engine, on the CPU."""
+import subprocess
+from pathlib import Path
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+def _run(tmp_path, name):
+    exe = tmp_path / name
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-pthread", "-I", str(ROOT / "wipems_gb300" / "csrc"), "-I",
+                        "/usr/local/cuda/include", "-o", str(exe), str(ROOT / "tests" / "glue" / f"{name}.cpp")],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout.endswith("ok\n"), r.stdout + r.stderr
+
+
+def test_device_buffer_after_a_failed_allocation(tmp_path):
+    """A buffer whose allocation failed holds nothing, so the next attempt
+    allocates again and no kernel gets a null pointer."""
+    _run(tmp_path, "memory_harness")

@@ -1220,16 +1220,6 @@ int fdtd_engine_checkpoint(fdtd_engine_t e, void* buf, uint64_t cap, uint64_t* s
 }
 
 namespace {
-// Device scratch of field dumps and readbacks, grown on demand.
-int grow_dump(fdtd_engine_s* e, size_t floats) {
-    if (e->dump.n >= floats) return FDTD_OK;
-    if (e->dump.p) {
-        e->device_bytes -= e->dump.n * sizeof(float);
-        e->dump.release();
-    }
-    return e->dump.alloc(floats, e->device_bytes, e->stream);
-}
-
 // Maps the pages of a large host destination before the device writes to it,
 // a share per thread.  A fresh array's pages do not exist yet, and faulting
 // them in one by one under the copy takes many times the copy: both fields of
@@ -1438,7 +1428,7 @@ int fdtd_engine_get_fields(fdtd_engine_t e, float* volt, float* curr) {
     // slab by slab through a packed array of at most 128 MB (at least a plane)
     const uint32_t slab = (uint32_t)std::min<size_t>(M[0], std::max<size_t>(1, ((size_t)32 << 20) / plane));
     int rc;
-    if ((rc = grow_dump(e, slab * plane))) return rc;
+    if ((rc = e->dump.grow(slab * plane, e->device_bytes, e->stream))) return rc;
     const int f = (2 + e->rot) % 3;
     for (int which = 0; which < 2; ++which) {
         float* dst = which ? curr : volt;
@@ -1502,7 +1492,7 @@ int fdtd_engine_dump_field(fdtd_engine_t e, const fdtd_dump_box* b, float* out, 
     CK(cudaSetDevice(e->device));
     int rc;
     if ((rc = start(e))) return rc;
-    if ((rc = grow_dump(e, 3 * total))) return rc;
+    if ((rc = e->dump.grow(3 * total, e->device_bytes, e->stream))) return rc;
     d.rot = e->rot;
     const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, 4096);
     k_dump_field<<<blocks, 256, 0, e->stream>>>(e->g, e->cur_V(), e->cur_I(), e->edges.p, d, e->dump.p);
@@ -1572,10 +1562,7 @@ int fdtd_engine_probe_now(fdtd_engine_t e, const fdtd_probe_desc* p, double* val
     if (ent.empty()) return FDTD_OK;
     CK(cudaSetDevice(e->device));
     uint64_t& tb = e->device_bytes;
-    if (e->now_entries.n < ent.size()) {
-        e->now_entries.release();
-        if ((rc = e->now_entries.alloc(ent.size(), tb, e->stream))) return rc;
-    }
+    if ((rc = e->now_entries.grow(ent.size(), tb, e->stream))) return rc;
     if (!e->now_misc.p && (rc = e->now_misc.alloc(4, tb, e->stream))) return rc;
     // now_misc: [0] the sum, [1] div = 0 (an integral), [2..3] first = {0, count} as ints
     double misc[4] = {0.0, 0.0, 0.0, 0.0};

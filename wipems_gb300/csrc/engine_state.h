@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "cop.h"
+#include "dev_buf.h"
 #include "fdtd_host.h"
 #include "kernels.cuh"
 #include "kernels_fused.cuh"
@@ -25,40 +26,6 @@ namespace wipems {
             return FDTD_ERR_CUDA;                                          \
         }                                                                  \
     } while (0)
-
-// Device buffer.  With a stream the memory comes from the device's
-// stream-ordered pool (cudaMallocAsync / cudaFreeAsync on that stream):
-// unlike cudaMalloc / cudaFree, neither synchronises the device, so a
-// server can create and destroy engines while other engines' work is in
-// flight.  The stream must outlive the buffer.
-template <class T>
-struct DevBuf {
-    T* p = nullptr;
-    size_t n = 0;
-    cudaStream_t s = nullptr;
-    ~DevBuf() { release(); }
-    void release() {
-        if (p) {
-            if (s) cudaFreeAsync(p, s);
-            else cudaFree(p);
-        }
-        p = nullptr;
-    }
-    int alloc(size_t count, uint64_t& total, cudaStream_t stream = nullptr) {
-        n = count;
-        s = stream;
-        if (count == 0) return FDTD_OK;
-        cudaError_t e = stream ? cudaMallocAsync(&p, count * sizeof(T), stream) : cudaMalloc(&p, count * sizeof(T));
-        if (e == cudaSuccess && stream) e = cudaStreamSynchronize(stream);  // usable from any stream from here on
-        if (e != cudaSuccess) {
-            p = nullptr;
-            set_error(std::string(stream ? "cudaMallocAsync: " : "cudaMalloc: ") + cudaGetErrorString(e));
-            return FDTD_ERR_NOMEM;
-        }
-        total += count * sizeof(T);
-        return FDTD_OK;
-    }
-};
 
 struct DevHalfBufs {
     DevBuf<uint8_t> idx;
