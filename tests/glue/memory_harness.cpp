@@ -4,15 +4,17 @@
 #include <cstdlib>
 #include <set>
 
-#include "dev_buf.h"
+#include <vector>
 
-static size_t g_limit = 0, g_used = 0;
+#include "readback.h"
+
+static size_t g_limit = 0;  // of one allocation
 static std::set<void*> g_live;
 static cudaError_t g_last = cudaSuccess;
 
 extern "C" {
 cudaError_t cudaMallocAsync(void** p, size_t bytes, cudaStream_t) {
-    if (g_used + bytes > g_limit) return g_last = cudaErrorMemoryAllocation;
+    if (bytes > g_limit) return g_last = cudaErrorMemoryAllocation;
     *p = std::malloc(bytes ? bytes : 1);
     g_live.insert(*p);
     return cudaSuccess;
@@ -66,6 +68,44 @@ int main() {
         CHECK(!b.p && b.n == 0);
     }
     CHECK(g_live.empty());
+    {  // the planes of a readback: all of them, fewer where memory is short, none
+        using wipems::readback_planes;
+        DevBuf<float> keep, once;
+        float* scratch = nullptr;
+        total = 0;
+        g_limit = 1 << 30;
+        CHECK(readback_planes(20, 1000, keep, once, total, st, &scratch) == 20 && scratch == keep.p && total == 80000);
+        CHECK(readback_planes(257, 257 * 257, keep, once, total, st, &scratch) == 257 && scratch == once.p);
+        CHECK(total == 80000 && keep.n == 20000);  // a large scratch is not the engine's
+        once.release();
+        CHECK(readback_planes(2000, 1 << 20, keep, once, total, st, &scratch) == 32 && scratch == once.p);
+        once.release();
+        g_limit = 4 * 257 * 257 * 60;
+        CHECK(readback_planes(257, 257 * 257, keep, once, total, st, &scratch) == 32 && scratch == keep.p);
+        keep.release();
+        total = 0;
+        g_limit = 4 * 257 * 257;
+        CHECK(readback_planes(257, 257 * 257, keep, once, total, st, &scratch) == 1 && scratch == keep.p);
+        g_limit = 1000;
+        keep.release();
+        CHECK(readback_planes(257, 257 * 257, keep, once, total, st, &scratch) == 0 && !keep.p && !once.p);
+        CHECK(cudaGetLastError() == cudaSuccess);
+    }
+    CHECK(g_live.empty());
+    for (int rot = 0; rot < 3; ++rot) {  // device axis a = operator axis (a + rot) % 3
+        const uint32_t M[3] = {3, 5, 7}, N[3] = {M[rot], M[(1 + rot) % 3], M[(2 + rot) % 3]};
+        std::vector<float> dev(105), out(105, -1.f);
+        uint32_t d[3];
+        for (d[0] = 0; d[0] < N[0]; ++d[0])
+            for (d[1] = 0; d[1] < N[1]; ++d[1])
+                for (d[2] = 0; d[2] < N[2]; ++d[2]) {
+                    uint32_t o[3];
+                    for (int a = 0; a < 3; ++a) o[(a + rot) % 3] = d[a];
+                    dev[(d[0] * N[1] + d[1]) * N[2] + d[2]] = (float)((o[0] * M[1] + o[1]) * M[2] + o[2]);
+                }
+        wipems::turn_axes(dev.data(), M, rot, out.data());
+        for (int k = 0; k < 105; ++k) CHECK(out[k] == (float)k);
+    }
     std::puts("ok");
     return 0;
 }

@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <new>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -23,6 +24,7 @@
 
 #include "engine_state.h"
 #include "launch.cuh"
+#include "readback.h"
 
 namespace wipems {
 namespace {
@@ -1420,15 +1422,40 @@ int fdtd_engine_energy(fdtd_engine_t e, double* energy) {
     return FDTD_OK;
 }
 
+// The fields without device scratch: a component's rows to a host array, axes
+// turned over there.
+static int get_fields_host(fdtd_engine_t e, float* volt, float* curr) {
+    const size_t n = (size_t)e->N[0] * e->N[1] * e->N[2];
+    const std::unique_ptr<float[]> tmp(e->rot ? new (std::nothrow) float[n] : nullptr);
+    if (e->rot && !tmp) {
+        set_error("fdtd_engine_get_fields: host allocation failed");
+        return FDTD_ERR_NOMEM;
+    }
+    for (int which = 0; which < 2; ++which) {
+        float* dst = which ? curr : volt;
+        for (int c = 0; c < 3 && dst; ++c, dst += n) {
+            const float* src = (which ? e->cur_I() : e->cur_V()) + e->dev_comp(c) * e->comp;
+            CK(cudaMemcpy2DAsync(tmp ? tmp.get() : dst, e->N[2] * sizeof(float), src, e->Nzp * sizeof(float),
+                                 e->N[2] * sizeof(float), (size_t)e->N[0] * e->N[1], cudaMemcpyDeviceToHost, e->stream));
+            CK(cudaStreamSynchronize(e->stream));
+            if (tmp) turn_axes(tmp.get(), e->N0, e->rot, dst);
+        }
+    }
+    return FDTD_OK;
+}
+
 int fdtd_engine_get_fields(fdtd_engine_t e, float* volt, float* curr) {
     if (!e) return FDTD_ERR_ARG;
     CK(cudaSetDevice(e->device));
     const uint32_t* M = e->N0;
     const size_t plane = (size_t)M[1] * M[2], n = plane * M[0];
-    // slab by slab through a packed array of at most 128 MB (at least a plane)
-    const uint32_t slab = (uint32_t)std::min<size_t>(M[0], std::max<size_t>(1, ((size_t)32 << 20) / plane));
+    // plane by plane of the first axis through a packed array, or turned over
+    // on the host where the device has no memory for one
+    DevBuf<float> once;
+    float* scratch = nullptr;
+    const uint32_t slab = readback_planes(M[0], plane, e->dump, once, e->device_bytes, e->stream, &scratch);
+    if (!slab) return get_fields_host(e, volt, curr);
     int rc;
-    if ((rc = e->dump.grow(slab * plane, e->device_bytes, e->stream))) return rc;
     const int f = (2 + e->rot) % 3;
     for (int which = 0; which < 2; ++which) {
         float* dst = which ? curr : volt;
@@ -1440,10 +1467,10 @@ int fdtd_engine_get_fields(fdtd_engine_t e, float* volt, float* curr) {
                 const uint32_t hi = std::min(M[0], lo + slab);
                 const dim3 grid((M[2] + 31) / 32, ((f == 0 ? hi - lo : M[1]) + 31) / 32,
                                 std::min(f == 0 ? M[1] : hi - lo, 65535u));
-                k_pack_field<<<grid, 256, 0, e->stream>>>(src, e->dump.p, (int)M[0], (int)M[1], (int)M[2], e->g.sx, e->Nzp,
+                k_pack_field<<<grid, 256, 0, e->stream>>>(src, scratch, (int)M[0], (int)M[1], (int)M[2], e->g.sx, e->Nzp,
                                                           e->rot, (int)lo, (int)hi);
                 if ((rc = check_launch())) return rc;
-                CK(cudaMemcpyAsync(dst + c * n + lo * plane, e->dump.p, (hi - lo) * plane * sizeof(float),
+                CK(cudaMemcpyAsync(dst + c * n + lo * plane, scratch, (hi - lo) * plane * sizeof(float),
                                    cudaMemcpyDeviceToHost, e->stream));
             }
         }

@@ -1,0 +1,41 @@
+// Host side of field readbacks: the device scratch they get and the order of
+// axes without one.
+#pragma once
+
+#include <algorithm>
+
+#include "dev_buf.h"
+
+namespace wipems {
+
+constexpr size_t kReadbackFloats = (size_t)32 << 20;  // scratch of a readback, at most (128 MB), and
+constexpr size_t kReadbackKept = (size_t)4 << 20;     // what of it an engine keeps for the next one (16 MB)
+
+// Planes (of `plane` floats each, at most `planes`) that a readback packs at
+// a time, with a scratch for them: `keep` if that is small, else `once`, which
+// the caller gives back.  Where memory is short fewer planes at a time, down
+// to one; 0 if there is not even that.
+inline uint32_t readback_planes(uint32_t planes, size_t plane, DevBuf<float>& keep, DevBuf<float>& once,
+                                uint64_t& kept_bytes, cudaStream_t st, float** scratch) {
+    uint64_t bytes = 0;  // of `once`: not the engine's
+    for (uint32_t n = (uint32_t)std::min<size_t>(planes, std::max<size_t>(1, kReadbackFloats / plane)); n > 0; n /= 2) {
+        const bool small = n * plane <= std::max(kReadbackKept, keep.n);
+        if ((small ? keep.grow(n * plane, kept_bytes, st) : once.grow(n * plane, bytes, st)) != FDTD_OK) continue;
+        *scratch = small ? keep.p : once.p;
+        return n;
+    }
+    return 0;
+}
+
+// One component from device axes to the operator's (device axis a = operator
+// axis (a + rot) % 3): s[N0][N1][N2] with N[a] = M[(a + rot) % 3], d[M0][M1][M2].
+inline void turn_axes(const float* s, const uint32_t M[3], int rot, float* d) {
+    uint32_t o[3];
+    const size_t N1 = M[(1 + rot) % 3], N2 = M[(2 + rot) % 3];
+    for (o[0] = 0; o[0] < M[0]; ++o[0])
+        for (o[1] = 0; o[1] < M[1]; ++o[1])
+            for (o[2] = 0; o[2] < M[2]; ++o[2])
+                *d++ = s[(o[rot % 3] * N1 + o[(1 + rot) % 3]) * N2 + o[(2 + rot) % 3]];
+}
+
+}  // namespace wipems
