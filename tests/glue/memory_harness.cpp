@@ -2,6 +2,7 @@
 // on demand: no GPU.
 #include <cstdio>
 #include <cstdlib>
+#include <new>
 #include <set>
 
 #include <vector>
@@ -37,6 +38,16 @@ const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 namespace wipems {
 void set_error(const std::string&) {}
 }
+
+static long g_news = -1;  // operator new calls before it throws (-1: never)
+void* operator new(size_t n) {
+    if (g_news == 0) throw std::bad_alloc();
+    if (g_news > 0) --g_news;
+    if (void* p = std::malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 #define CHECK(x)                                              \
     do {                                                      \
@@ -105,6 +116,15 @@ int main() {
                 }
         wipems::turn_axes(dev.data(), M, rot, out.data());
         for (int k = 0; k < 105; ++k) CHECK(out[k] == (float)k);
+    }
+    {  // pages are touched whatever the host's memory allows; nothing is thrown
+        std::vector<char> dst((size_t)16 << 20, 1);
+        for (long news : {0L, 1L, 2L, 5L, -1L}) {
+            g_news = news;
+            wipems::touch_pages(dst.data() + 3, dst.size() - 7);
+            g_news = -1;
+            CHECK(dst[2] == 1 && dst[3] == 0 && dst[dst.size() - 4] == 1);
+        }
     }
     std::puts("ok");
     return 0;

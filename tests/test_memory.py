@@ -18,5 +18,6 @@ def _run(tmp_path, name):
 def test_device_buffer_after_a_failed_allocation(tmp_path):
     """A buffer whose allocation failed holds nothing, so the next attempt
     allocates again and no kernel gets a null pointer; a readback takes the
-    scratch it can get, down to none, and then turns the axes over here."""
+    scratch it can get, down to none, and then turns the axes over here; the
+    threads that map its pages may fail to start at any of their allocations."""
     _run(tmp_path, "memory_harness")

@@ -17,8 +17,6 @@
 #include <memory>
 #include <new>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 
@@ -1220,34 +1218,6 @@ int fdtd_engine_checkpoint(fdtd_engine_t e, void* buf, uint64_t cap, uint64_t* s
     CK(cudaStreamSynchronize(e->stream));
     return FDTD_OK;
 }
-
-namespace {
-// Maps the pages of a large host destination before the device writes to it,
-// a share per thread.  A fresh array's pages do not exist yet, and faulting
-// them in one by one under the copy takes many times the copy: both fields of
-// 257^3 lines (408 MB) took 335 ms to read, 6.4 ms with their pages mapped by
-// 16 threads first.  Small arrays (over the allocator's usual threshold for
-// fresh pages) are touched by the calling thread alone.
-void touch_pages(void* p, size_t bytes) {
-    if (bytes < (size_t)256 << 10) return;
-    const size_t page = 4096;
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned nt = (unsigned)std::max<size_t>(1, std::min<size_t>(std::min(hw, 16u), bytes >> 21));
-    auto part = [=](unsigned k) {
-        volatile char* b = static_cast<volatile char*>(p);
-        const size_t lo = bytes / nt * k, hi = k + 1 == nt ? bytes : bytes / nt * (k + 1);
-        for (size_t o = lo; o < hi; o += page) b[o] = 0;
-        if (hi > lo) b[hi - 1] = 0;
-    };
-    std::vector<std::thread> th;
-    try {
-        for (unsigned k = 1; k < nt; ++k) th.emplace_back(part, k);
-    } catch (const std::system_error&) {  // fewer threads: the copy maps the rest
-    }
-    part(0);
-    for (std::thread& t : th) t.join();
-}
-}  // namespace
 
 // Restore validates the whole blob -- header, sample count and every part's
 // size against this engine, and the blob's length -- before it changes
