@@ -1392,8 +1392,8 @@ int fdtd_engine_energy(fdtd_engine_t e, double* energy) {
     return FDTD_OK;
 }
 
-// The fields without device scratch: a component's rows to a host array, axes
-// turned over there.
+// The fields without device scratch: rows to the host as they are, axes turned
+// over there.
 static int get_fields_host(fdtd_engine_t e, float* volt, float* curr) {
     const size_t n = (size_t)e->N[0] * e->N[1] * e->N[2];
     const std::unique_ptr<float[]> tmp(e->rot ? new (std::nothrow) float[n] : nullptr);
@@ -1403,14 +1403,23 @@ static int get_fields_host(fdtd_engine_t e, float* volt, float* curr) {
     }
     for (int which = 0; which < 2; ++which) {
         float* dst = which ? curr : volt;
-        for (int c = 0; c < 3 && dst; ++c, dst += n) {
-            const float* src = (which ? e->cur_I() : e->cur_V()) + e->dev_comp(c) * e->comp;
-            CK(cudaMemcpy2DAsync(tmp ? tmp.get() : dst, e->N[2] * sizeof(float), src, e->Nzp * sizeof(float),
-                                 e->N[2] * sizeof(float), (size_t)e->N[0] * e->N[1], cudaMemcpyDeviceToHost, e->stream));
+        if (!dst) continue;
+        const float* src = which ? e->cur_I() : e->cur_V();
+        touch_pages(dst, 3 * n * sizeof(float));
+        const size_t row = e->N[2] * sizeof(float), rows = (size_t)e->N[0] * e->N[1];
+        if (!tmp) {
+            CK(cudaMemcpy2DAsync(dst, row, src, e->Nzp * sizeof(float), row, 3 * rows, cudaMemcpyDeviceToHost,
+                                 e->stream));
+            continue;
+        }
+        for (int c = 0; c < 3; ++c) {
+            CK(cudaMemcpy2DAsync(tmp.get(), row, src + e->dev_comp(c) * e->comp, e->Nzp * sizeof(float), row, rows,
+                                 cudaMemcpyDeviceToHost, e->stream));
             CK(cudaStreamSynchronize(e->stream));
-            if (tmp) turn_axes(tmp.get(), e->N0, e->rot, dst);
+            turn_axes(tmp.get(), e->N0, e->rot, dst + c * n);
         }
     }
+    CK(cudaStreamSynchronize(e->stream));
     return FDTD_OK;
 }
 
@@ -1418,31 +1427,31 @@ int fdtd_engine_get_fields(fdtd_engine_t e, float* volt, float* curr) {
     if (!e) return FDTD_ERR_ARG;
     CK(cudaSetDevice(e->device));
     const uint32_t* M = e->N0;
-    const size_t plane = (size_t)M[1] * M[2], n = plane * M[0];
-    // plane by plane of the first axis through a packed array, or turned over
-    // on the host where the device has no memory for one
+    const size_t plane = (size_t)M[1] * M[2];
+    // small arrays in the operator's axes: the copies alone (26 x 11 x 32
+    // lines 28 us, packed first 39; 41^3 lines 70 us, packed 49)
+    if (e->rot == 0 && 3 * M[0] * plane * sizeof(float) < kFreshBytes) return get_fields_host(e, volt, curr);
+    // planes of the first axis, of all components, through a packed array, or
+    // turned over on the host where the device has no memory for one
     DevBuf<float> once;
     float* scratch = nullptr;
-    const uint32_t slab = readback_planes(M[0], plane, e->dump, once, e->device_bytes, e->stream, &scratch);
+    const uint32_t planes = 3 * M[0], slab = readback_planes(planes, plane, e->dump, once, e->device_bytes, e->stream, &scratch);
     if (!slab) return get_fields_host(e, volt, curr);
     int rc;
     const int f = (2 + e->rot) % 3;
     for (int which = 0; which < 2; ++which) {
         float* dst = which ? curr : volt;
         if (!dst) continue;
-        touch_pages(dst, 3 * n * sizeof(float));
-        for (int c = 0; c < 3; ++c) {
-            const float* src = (which ? e->cur_I() : e->cur_V()) + e->dev_comp(c) * e->comp;
-            for (uint32_t lo = 0; lo < M[0]; lo += slab) {
-                const uint32_t hi = std::min(M[0], lo + slab);
-                const dim3 grid((M[2] + 31) / 32, ((f == 0 ? hi - lo : M[1]) + 31) / 32,
-                                std::min(f == 0 ? M[1] : hi - lo, 65535u));
-                k_pack_field<<<grid, 256, 0, e->stream>>>(src, scratch, (int)M[0], (int)M[1], (int)M[2], e->g.sx, e->Nzp,
-                                                          e->rot, (int)lo, (int)hi);
-                if ((rc = check_launch())) return rc;
-                CK(cudaMemcpyAsync(dst + c * n + lo * plane, scratch, (hi - lo) * plane * sizeof(float),
-                                   cudaMemcpyDeviceToHost, e->stream));
-            }
+        touch_pages(dst, planes * plane * sizeof(float));
+        for (uint32_t lo = 0; lo < planes; lo += slab) {
+            const uint32_t hi = std::min(planes, lo + slab);
+            const dim3 grid((M[2] + 31) / 32, ((f == 0 ? hi - lo : M[1]) + 31) / 32,
+                            std::min(f == 0 ? M[1] : hi - lo, 65535u));
+            k_pack_field<<<grid, 256, 0, e->stream>>>(which ? e->cur_I() : e->cur_V(), scratch, (int)M[0], (int)M[1],
+                                                      (int)M[2], e->comp, e->g.sx, e->Nzp, e->rot, (int)lo, (int)hi);
+            if ((rc = check_launch())) return rc;
+            CK(cudaMemcpyAsync(dst + lo * plane, scratch, (hi - lo) * plane * sizeof(float), cudaMemcpyDeviceToHost,
+                               e->stream));
         }
     }
     CK(cudaStreamSynchronize(e->stream));

@@ -630,32 +630,34 @@ static __global__ void k_rlc(const DevGrid g, RlcSet rs, int ts_off) {
 }
 
 // ----------------------------------------------------------- field readback
-// Planes lo <= o0 < hi of one component of a field array, from device axes
-// and padded rows to the operator's axes without padding
-// (out[o0 - lo][o1][o2]).  rot: device axis a = operator axis (a + rot) % 3,
-// so the two layouts' fastest axes differ when rot != 0 and 32 x 32 tiles
-// turn over in shared memory: both sides move whole 128-byte rows.  A tile
-// spans the operator's fastest axis and the one that is fastest on the
-// device; the third runs over blockIdx.z.  Bandwidth-bound, and a small part
-// of the copy to the host that follows; the same reordering done on the host
-// node by node took 10.7 ms for 132 x 98 x 76 lines, against 0.8 ms for
-// packing and copying.
+// Planes lo <= p < hi of a field array, from device axes and padded rows to
+// the operator's axes without padding: plane p is plane p % M0 of the
+// operator's component p / M0, out[p - lo][M1][M2].  Device axis a = operator
+// axis (a + rot) % 3, so the two layouts' fastest axes differ when rot != 0
+// and 32 x 32 tiles turn over in shared memory: both sides move whole
+// 128-byte rows.  A tile spans the operator's fastest axis and the one that
+// is fastest on the device; the third runs over blockIdx.z.  Bandwidth-bound,
+// and a small part of the copy to the host that follows; the same reordering
+// done on the host node by node took 10.7 ms for 132 x 98 x 76 lines, against
+// 0.8 ms for packing and copying.  One launch takes all components: a launch
+// and a copy per component took 94 us for 12^3 lines, now 36.
 static __global__ void __launch_bounds__(256) k_pack_field(const float* __restrict__ src, float* __restrict__ out,
-                                                           int M0, int M1, int M2, long long sx, int Nzp, int rot,
-                                                           int lo, int hi) {
+                                                           int M0, int M1, int M2, long long comp, long long sx,
+                                                           int Nzp, int rot, int lo, int hi) {
     __shared__ float tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int f = (2 + rot) % 3;  // the operator's axis that is fastest on the device
+    const int f = (2 + rot) % 3;  // the operator's axis that is fastest on the device (0: with p)
     if (f == 2) {  // same fastest axis: rows only lose their padding
         const int o2 = blockIdx.x * 32 + tx, o1 = blockIdx.y * 32 + ty;
         if (o2 >= M2) return;
-        for (int o0 = lo + (int)blockIdx.z; o0 < hi; o0 += gridDim.z)
+        for (int p = lo + (int)blockIdx.z; p < hi; p += gridDim.z) {
+            const float* s = src + p / M0 * comp + p % M0 * sx;
             for (int k = 0; k < 32 && o1 + k < M1; k += 8)
-                out[((long long)(o0 - lo) * M1 + o1 + k) * M2 + o2] =
-                    src[(long long)o0 * sx + (long long)(o1 + k) * Nzp + o2];
+                out[((long long)(p - lo) * M1 + o1 + k) * M2 + o2] = s[(long long)(o1 + k) * Nzp + o2];
+        }
         return;
     }
-    const int beg[2] = {lo, 0}, end[2] = {hi, M1};  // ranges of the operator's axes 0 and 1
+    const int beg[2] = {lo, 0}, end[2] = {hi, M1};  // ranges of p and the operator's axis 1
     const int a = 1 - f;
     const int of = beg[f] + (int)blockIdx.y * 32, o2 = (int)blockIdx.x * 32;
     for (int oa = beg[a] + (int)blockIdx.z; oa < end[a]; oa += gridDim.z) {
@@ -665,8 +667,9 @@ static __global__ void __launch_bounds__(256) k_pack_field(const float* __restri
             o[f] = of + tx;
             o[2] = o2 + ty + k;
             if (o[f] < end[f] && o[2] < M2) {
-                for (int c = 0; c < 3; ++c) d[c] = o[(c + rot) % 3];
-                tile[ty + k][tx] = src[(long long)d[0] * sx + (long long)d[1] * Nzp + d[2]];
+                const int n = o[0] / M0, q[3] = {o[0] - n * M0, o[1], o[2]};
+                for (int c = 0; c < 3; ++c) d[c] = q[(c + rot) % 3];
+                tile[ty + k][tx] = src[(n - rot + 3) % 3 * comp + (long long)d[0] * sx + (long long)d[1] * Nzp + d[2]];
             }
         }
         __syncthreads();
