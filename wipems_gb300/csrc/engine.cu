@@ -466,8 +466,6 @@ int reset_state(fdtd_engine_s* e) {
     for (DevBuf<float>* b : {&e->AVx, &e->LVx, &e->AIx, &e->LIx})
         if (b->p) CK(cudaMemsetAsync(b->p, 0, b->n * sizeof(float), s));
     CK(cudaMemsetAsync(e->ctl.p, 0, 4 * sizeof(int), s));
-    CK(cudaMemsetAsync(e->ticket.p, 0, sizeof(unsigned), s));
-    if (e->res_ll.p) CK(cudaMemsetAsync(e->res_ll.p, 0, e->res_ll.n * sizeof(ulonglong2), s));
     if (e->d_fd.p) CK(cudaMemsetAsync(e->d_fd.p, 0, e->d_fd.n * sizeof(double), s));
     if (e->mur_buf.p) CK(cudaMemsetAsync(e->mur_buf.p, 0, e->mur_buf.n * sizeof(float), s));
     if (e->rlc_state.p) CK(cudaMemsetAsync(e->rlc_state.p, 0, e->rlc_state.n * sizeof(float), s));
@@ -627,6 +625,7 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
     if ((rc = e->ctl.alloc(4, tot, e->stream)) || (rc = e->d_eacc.alloc(4, tot, e->stream)) ||
         (rc = e->d_energy_tmp.alloc(2, tot, e->stream)) || (rc = e->ticket.alloc(1, tot, e->stream)))
         return rc;
+    CK(cudaMemsetAsync(e->ticket.p, 0, sizeof(unsigned), e->stream));  // every launch leaves it at zero
     // energy segments: one float pair per (x < Nx-1, y < Ny-1, 32-node z tile)
     const int nzt = ((int)e->N[2] - 1 + 31) / 32;
     if ((rc = e->eseg.alloc((size_t)(e->N[0] - 1) * (e->N[1] - 1) * (size_t)nzt, tot, e->stream)) ||
@@ -1287,8 +1286,6 @@ int fdtd_engine_restore(fdtd_engine_t e, const void* buf, uint64_t size) {
         if (b) CK(cudaMemcpyAsync(q.p, o, b, cudaMemcpyHostToDevice, e->stream));
         o += b;
     }
-    // numTS may go back: no exchange word of a later timestep may stay
-    if (e->res_ll.p) CK(cudaMemsetAsync(e->res_ll.p, 0, e->res_ll.n * sizeof(ulonglong2), e->stream));
     CK(cudaStreamSynchronize(e->stream));
     e->ts = h.ts;
     e->done = h.done != 0;

@@ -143,6 +143,7 @@ struct fdtd_engine_s {
     const void* res_kernel = nullptr;
     int res_smem = 0, res_threads = 0, res_samples = 0;  // samples one run can hold
     DevBuf<ulonglong2> res_ll;             // exchange pairs
+    uint32_t res_tag = 0;                  // the largest tag stored in them
     DevBuf<float> res_pval, res_fdval;     // probe entry values of a run's samples / frequency-domain steps
     DevBuf<float2> res_seg;                // their energy segments and plane sums
     DevBuf<double2> res_plane;

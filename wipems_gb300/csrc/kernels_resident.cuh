@@ -5,7 +5,8 @@
 // owns a box of nodes and keeps its voltages, currents and tuple indices in
 // shared memory from the first to the last timestep of the run.  A warp
 // takes 32 z-nodes of a row at a time.  What a box needs of its neighbours
-// goes through global memory (L2) as 64-bit words {value, timestep}: the
+// goes through global memory (L2) as 64-bit words {value, tag}, the tag
+// counting the timesteps of all runs of the engine (numTS may go back): the
 // reader polls the very word it needs, so an exchange costs one store and
 // one load, no fence, flag or barrier.  Words of even and odd timesteps lie
 // in two buffers: a node's word of timestep n + 2 is stored only after that
@@ -69,6 +70,7 @@ struct ResArgs {
     int p[3];                // boxes per axis
     int ne[3];               // extent of the voltage update
     int ts0, nsteps;         // numTS at the start, timesteps of this run
+    uint32_t tag0;           // tags below and up to this one are of earlier runs
     int interval;            // samples after every interval-th timestep (0 = none)
     ulonglong2* ll;          // exchange pairs: [V, I][even, odd][x cuts, y cuts, z cuts]
     long long ll_pairs;      // pairs per field and parity
@@ -449,7 +451,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
     int samples = 0, fds = 0;
     for (int k = 0; k < a.nsteps; ++k) {
         const int ts = a.ts0 + k;
-        const uint32_t tag = (uint32_t)ts + 1u;  // of this timestep's new values
+        const uint32_t tag = a.tag0 + (uint32_t)k + 1u;  // of this timestep's new values
         ulonglong2* llV = a.ll + (long long)(tag & 1u) * a.ll_pairs;
         ulonglong2* llI = a.ll + (long long)(2u + (tag & 1u)) * a.ll_pairs;
         const ulonglong2* llJ = a.ll + (long long)(2u + ((tag & 1u) ^ 1u)) * a.ll_pairs;  // old currents
@@ -486,9 +488,9 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
                         i1zm = g.I[C + go - 1];
                     }
                 } else {
-                    if (nx) ll_wait(llJ + (xl + y * a.cov[2] + z), (uint32_t)ts, i1xm, i2xm, ok);
-                    if (ny) ll_wait(llJ + (yl + x * a.cov[2] + z), (uint32_t)ts, i0ym, i2ym, ok);
-                    if (nz) ll_wait(llJ + (zl + x * a.cov[1] + y), (uint32_t)ts, i0zm, i1zm, ok);
+                    if (nx) ll_wait(llJ + (xl + y * a.cov[2] + z), tag - 1u, i1xm, i2xm, ok);
+                    if (ny) ll_wait(llJ + (yl + x * a.cov[2] + z), tag - 1u, i0ym, i2ym, ok);
+                    if (nz) ll_wait(llJ + (zl + x * a.cov[1] + y), tag - 1u, i0zm, i1zm, ok);
                 }
             }
             if (z < zE && (e.x & RT_ROW)) {

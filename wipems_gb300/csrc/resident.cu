@@ -51,6 +51,7 @@ constexpr size_t kSampleBytes = (size_t)16 << 20;  // of a run's energy segments
 constexpr int kMaxRunSamples = 64;
 constexpr int kMaxRunFd = 256;
 constexpr uint32_t kMaxRun = 1024;  // timesteps of one launch
+constexpr uint32_t kMaxTag = 1u << 30;  // the exchange words are cleared above it
 
 }  // namespace
 
@@ -172,6 +173,12 @@ int launch_resident(fdtd_engine_s* e, uint32_t n, cudaStream_t st) {
     ResArgs a = e->ra;
     a.ts0 = (int)e->ts;
     a.nsteps = (int)n;
+    if (e->res_tag > kMaxTag) {
+        CK(cudaMemsetAsync(e->res_ll.p, 0, e->res_ll.n * sizeof(ulonglong2), st));
+        e->res_tag = 0;
+    }
+    a.tag0 = e->res_tag;
+    e->res_tag += n;
     void* args[] = {&e->g, &a, &e->ps};
     CK(cudaLaunchCooperativeKernel(e->res_kernel, dim3((unsigned)(a.p[0] * a.p[1] * a.p[2])),
                                    dim3((unsigned)e->res_threads), args, (size_t)e->res_smem, st));
