@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from wipems_gb300 import CompressedOperator, Engine, Operator, Scene
-from wipems_gb300.fdtd import BC_PEC, BC_PMC, BC_PML
+from wipems_gb300.fdtd import BC_MUR, BC_PEC, BC_PMC, BC_PML
 
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("libs")]
 
@@ -88,3 +88,20 @@ def test_samples_without_energies(nprobe, interval):
         e.iterate(200)
     _same(*es)
     assert es[0].samples().values.shape == (207 // interval + 1, nprobe)
+
+
+@pytest.mark.parametrize("wall,single", [(BC_PEC, 3), (BC_PML, 3), (BC_MUR, 2)])
+def test_route_by_length(wall, single):
+    """A call of one timestep runs on the half-step kernels (two launches and
+    the counter's) unless Mur launches would come beside them; longer calls
+    run resident.  Mixed calls give the same bits as the two-pass kernels."""
+    cop = CompressedOperator(Operator(_scene((33, 30, 41), wall)))
+    es = [Engine(cop, max_timesteps=400, probe_interval=40, kernel=k) for k in ("auto", "tma")]
+    launches = {}
+    for steps in (1, 1, 2, 1, 30, 1, 1, 64, 1):
+        for e in es:
+            e.iterate(steps)
+        launches.setdefault(steps, set()).add(es[0].last_timing()[1])
+    # the first call also takes the sample of numTS 0
+    assert launches[1] == {single, single + 1} and launches[2] == {2} and launches[64] <= {2, 3}
+    _same(*es)

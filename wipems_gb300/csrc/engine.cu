@@ -1061,7 +1061,12 @@ int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
     const bool fd_on = e->fd_interval && !e->h_freq.empty() && e->ps.nprobe;
     uint32_t left = n;
     while (left > 0) {
-        if (e->resident) {
+        // A single timestep pays for a whole trip of the state into shared memory
+        // and back: without Mur or RLC launches beside the half-steps those are
+        // faster (us per call, resident / half-steps: 65^3 PEC 40 / 40, 91^3 49 /
+        // 46, 102^3 61 / 52, 65 x 71 x 61 dispersive 49 / 44; with Mur 51 x 42 x 61
+        // 41 / 56).  Two timesteps are faster resident on all of these.
+        if (e->resident && (left > 1 || e->mur.nface || e->rlc.count)) {
             const uint32_t run = resident_run(e, left);
             if ((rc = launch_resident(e, run, e->stream))) return rc;
             e->ts += run;
