@@ -3,7 +3,7 @@ fields of every timestep from memory: the same bits."""
 import numpy as np
 import pytest
 
-from wipems_gb300 import CompressedOperator, Engine, Operator, Scene
+from wipems_gb300 import Batch, CompressedOperator, Engine, Operator, Scene
 from wipems_gb300.fdtd import BC_MUR, BC_PEC, BC_PMC, BC_PML
 
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("libs")]
@@ -105,3 +105,23 @@ def test_route_by_length(wall, single):
     # the first call also takes the sample of numTS 0
     assert launches[1] == {single, single + 1} and launches[2] == {2} and launches[64] <= {2, 3}
     _same(*es)
+
+
+def test_batched_jobs_hold_no_resident_buffers():
+    """Jobs that a batch keeps in its own kernels get no buffers of resident
+    runs; a default engine gets them with its first run."""
+    cop = CompressedOperator(Operator(_scene((33, 33, 33))))
+    for kernel in ("tma", "auto"):
+        es = [Engine(cop, max_timesteps=300, kernel=kernel) for _ in range(16)]
+        for e in es:
+            e.energy()  # nothing to do with stepping
+        b0 = Batch(es[:1], bin_mib=64)  # starts the engine: probes and samples
+        base = es[0].stats()["device_bytes"]
+        b = Batch(es)
+        b.iterate(20)
+        assert b.stats()["num_bins"] == 1
+        assert {e.stats()["device_bytes"] for e in es} == {base}
+        es[0].iterate(20)
+        assert (es[0].stats()["device_bytes"] > base) == (kernel == "auto")
+        for e in (b0, b, *es):
+            e.close()

@@ -226,13 +226,19 @@ int split_jobs(std::vector<fdtd_engine_s*>& batched, std::vector<fdtd_engine_s*>
     std::vector<fdtd_engine_s*> fit, rest;
     double sum = 0.0;
     for (fdtd_engine_s* e : batched) {
-        if (e->E.idx16 && e->H.idx16 && e->end_crit == 0.0)
-            if (int rc = setup_resident(e)) return rc;
-        (e->res_ready && e->end_crit == 0.0 ? fit : rest).push_back(e);
-        if (fit.size() && fit.back() == e) sum += resident_us(e);
+        const bool may = e->E.idx16 && e->H.idx16 && e->end_crit == 0.0;
+        if (may)
+            if (int rc = plan_resident(e)) return rc;
+        (may && e->res_fits ? fit : rest).push_back(e);
+        if (may && e->res_fits) sum += resident_us(e);
     }
     const bool all = sum <= batched_us(fit, XC);
-    for (fdtd_engine_s* e : fit) (all || resident_us(e) < nodes_of(e) / 58e3 ? resident : rest).push_back(e);
+    for (fdtd_engine_s* e : fit) {
+        const bool res = all || resident_us(e) < nodes_of(e) / 58e3;
+        if (res)  // only these get the buffers of resident runs
+            if (int rc = setup_resident(e)) return rc;
+        (res && e->res_ready ? resident : rest).push_back(e);
+    }
     double alone = 0.0;
     bool may = true;
     for (const fdtd_engine_s* e : rest) {

@@ -279,8 +279,8 @@ int start(fdtd_engine_s* e) {
         if ((rc = upload_probes(e))) return rc;
         e->started = true;
         if (e->res_candidate) {
-            if ((rc = setup_resident(e))) return rc;
-            e->resident = e->res_ready;
+            if ((rc = plan_resident(e))) return rc;
+            e->resident = e->res_fits;
         }
         if (e->interval && e->use_graphs && !e->resident && (rc = build_chunk_graph(e))) return rc;
     }
@@ -1059,6 +1059,11 @@ int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
     CK(cudaEventRecord(e->ev0, e->stream));
     if ((rc = start(e))) return rc;
     const bool fd_on = e->fd_interval && !e->h_freq.empty() && e->ps.nprobe;
+    if (e->resident && n > 0 && !e->res_ready) {
+        if ((rc = setup_resident(e))) return rc;
+        e->resident = e->res_ready;
+        if (!e->resident && e->interval && e->use_graphs && (rc = build_chunk_graph(e))) return rc;
+    }
     uint32_t left = n;
     while (left > 0) {
         // A single timestep pays for a whole trip of the state into shared memory

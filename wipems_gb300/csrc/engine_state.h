@@ -138,7 +138,8 @@ struct fdtd_engine_s {
     FusedMaps fmaps{};
     // resident timesteps (kernels_resident.cuh): runs of timesteps with the
     // fields in shared memory, back in V / I at the end of each run
-    bool res_candidate = false, res_ready = false, resident = false;  // ready: set up; resident: own runs use it
+    bool res_planned = false, res_fits = false;  // plan_resident has run; the grid fits
+    bool res_candidate = false, res_ready = false, resident = false;  // ready: buffers there; resident: own runs use it
     ResArgs ra{};
     const void* res_kernel = nullptr;
     int res_smem = 0, res_threads = 0, res_samples = 0;  // samples one run can hold
@@ -208,7 +209,8 @@ inline int auto_x_chunk(const std::vector<const uint32_t*>& lines, uint64_t resi
 // resident.cu
 // boxes per axis, at most `blocks` of at most `nodes`; false if the grid does not fit
 bool resident_plan(const int cov[3], const bool mur[3], int blocks, int nodes, int p[3]);
-int setup_resident(fdtd_engine_s* e);  // sets e->res_ready if the grid fits
+int plan_resident(fdtd_engine_s* e);   // sets e->res_fits if the grid fits: no device memory yet
+int setup_resident(fdtd_engine_s* e);  // sets e->res_ready if it does and the memory was there
 uint32_t resident_run(const fdtd_engine_s* e, uint32_t n);  // timesteps the next launch can take, at most n
 int launch_resident(fdtd_engine_s* e, uint32_t n, cudaStream_t st);  // n timesteps and their samples
 

@@ -88,8 +88,9 @@ bool resident_plan(const int cov[3], const bool mur[3], int blocks, int nodes, i
     return best < 1e30;
 }
 
-int setup_resident(fdtd_engine_s* e) {
-    if (e->res_ready) return FDTD_OK;
+int plan_resident(fdtd_engine_s* e) {
+    if (e->res_planned) return FDTD_OK;
+    e->res_planned = true;
     int sms = 0, coop = 0, smem = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->device));
@@ -135,15 +136,23 @@ int setup_resident(fdtd_engine_s* e) {
     a.d_err = e->p_err();
     a.seg_stride = (long long)(e->N[0] - 1) * (e->N[1] - 1) * e->g.nzt;
     e->res_samples = (int)std::max<size_t>(1, std::min<size_t>(kMaxRunSamples, kSampleBytes / (8 * a.seg_stride)));
+    e->res_fits = true;
+    return FDTD_OK;
+}
+
+int setup_resident(fdtd_engine_s* e) {
+    if (int rc = plan_resident(e)) return rc;
+    if (e->res_ready || !e->res_fits) return FDTD_OK;
+    ResArgs& a = e->ra;
+    const size_t samples = e->interval ? e->res_samples : 0, esamples = e->energy_on_probe ? samples : 0;
     uint64_t& tot = e->device_bytes;
     const uint64_t before = tot;
     if (e->res_ll.alloc(std::max<long long>(1, 4 * a.ll_pairs), tot, e->stream) ||
-        e->res_pval.alloc(std::max<size_t>(1, entries * e->res_samples), tot, e->stream) ||
-        (fd && e->res_fdval.alloc(std::max<size_t>(1, entries * kMaxRunFd), tot, e->stream)) ||
-        e->res_seg.alloc(a.seg_stride * e->res_samples, tot, e->stream) ||
-        e->res_plane.alloc((size_t)(e->N[0] - 1) * e->res_samples, tot, e->stream)) {
+        e->res_pval.alloc(a.nentry * samples, tot, e->stream) ||
+        e->res_fdval.alloc(a.fd_interval ? (size_t)a.nentry * kMaxRunFd : 0, tot, e->stream) ||
+        e->res_seg.alloc(a.seg_stride * esamples, tot, e->stream) ||
+        e->res_plane.alloc((e->N[0] - 1) * esamples, tot, e->stream)) {
         // no memory left for it: the half-step kernels need none
-        cudaGetLastError();
         e->res_ll.release();
         e->res_pval.release();
         e->res_fdval.release();
@@ -155,7 +164,7 @@ int setup_resident(fdtd_engine_s* e) {
     a.ll = e->res_ll.p;
     a.pval = e->res_pval.p;
     a.fdval = e->res_fdval.p;
-    a.eseg = e->energy_on_probe ? e->res_seg.p : nullptr;
+    a.eseg = e->res_seg.p;
     CK(cudaMemsetAsync(e->res_ll.p, 0, e->res_ll.n * sizeof(ulonglong2), e->stream));
     e->res_ready = true;
     return FDTD_OK;
