@@ -1,4 +1,5 @@
-"""Host-side memory handling of the engine, on the CPU."""
+"""Host-side parts of the engine, on the CPU: memory and error words."""
+import ctypes
 import subprocess
 from pathlib import Path
 
@@ -21,3 +22,13 @@ def test_device_buffer_after_a_failed_allocation(tmp_path):
     scratch it can get, down to none, and then turns the axes over here; the
     threads that map its pages may fail to start at any of their allocations."""
     _run(tmp_path, "memory_harness")
+
+
+def test_error_words(libs):
+    """Each bounded device wait is reported as what it was."""
+    from wipems_gb300 import _abi
+    L = ctypes.CDLL(str(_abi.LIB_PATH))
+    decode = L._ZN6wipems19engine_decode_errorEi  # wipems::engine_decode_error(int)
+    for err, text in [(4, "TMA copy"), (8, "resident run"), (1, "ring overflow"), (2, "not finite")]:
+        assert decode(err) != 0 and text in _abi.last_error()
+    assert decode(4) == decode(8) != decode(1) and decode(0) == 0

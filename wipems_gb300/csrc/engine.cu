@@ -299,6 +299,11 @@ int decode_error(int err) {
         set_error("a bounded device wait gave up: a TMA copy did not complete in time");
         return FDTD_ERR_TIMEOUT;
     }
+    if (err & 8) {
+        set_error("a bounded device wait gave up: the exchange between the blocks of a resident run did not complete "
+                  "in time");
+        return FDTD_ERR_TIMEOUT;
+    }
     if (err & 1) {
         set_error("probe sample ring overflow: raise max_timesteps");
         return FDTD_ERR_STATE;

@@ -198,7 +198,8 @@ struct ProbeSet {
     double* ring;               // [cap][row_doubles]: ts, energy, values...
     int cap;
     int* d_nsamp;               // samples written
-    int* d_err;                 // error word (ring overflow, non-finite)
+    int* d_err;                 // error word: 1 ring overflow, 2 non-finite, 4 / 8 a wait
+                                // for a TMA copy / a resident run's exchange ran out
     int* d_done;                // end criterion met (0 / 1)
     double end_crit;            // > 0: stop once energy <= end_crit * max energy
     int stop_ts;                // > 0 (with end_crit): stop at this numTS

@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_resident(const DevGrid g, const
             __syncthreads();
         }
     }
-    if (!ok) atomicOr(a.d_err, 4);
+    if (!ok) atomicOr(a.d_err, 8);
     for (int r = warp; r < rows; r += nwarps) {
         const int x = r / by, y = r - x * by;
         const long long go = g0 + (long long)x * g.sx + (long long)y * g.Nzp;
