@@ -46,26 +46,31 @@ def tune(cop, stages=DEFAULT_STAGES, xchunks=DEFAULT_XCHUNK, steps: int = 30, de
     from ._abi import FdtdError
     from .fdtd import Engine
     table = []
-    for k in ("auto", *kernels):
-        own = k == "auto"
+
+    def candidate(k, ty, s, xc, own=False) -> bool:
+        try:
+            eng = Engine(cop, device=device, stages=s, x_chunk=xc, max_timesteps=2 * steps + 64, kernel=k, tile_y=ty)
+        except FdtdError:
+            return False  # kernel not applicable to this grid
+        eng.iterate(min(steps, 16))  # warm-up, graph instantiation
+        eng.reset()
+        eng.iterate(steps)
+        ms, _ = eng.last_timing()
+        tile = 0 if own else eng.stats()["tile_y"]
+        eng.close()
+        table.append(dict(kernel=k, tile_y=tile, stages=s, x_chunk=xc, ms_step=ms / steps))
+        if verbose:
+            print(f"kernel={k:5s} tile_y={tile} stages={s} x_chunk={xc:3d}  {ms / steps * 1e3:8.1f} us/step",
+                  flush=True)
+        return True
+
+    candidate("auto", 0, 0, 0, own=True)
+    for k in kernels:
         for ty in (tile_ys if k == "tma" else (0,)):
-            for s in (0,) if own else stages:
-                for xc in (0,) if own else xchunks:
-                    try:
-                        eng = Engine(cop, device=device, stages=s, x_chunk=xc, max_timesteps=2 * steps + 64,
-                                     kernel=k, tile_y=ty)
-                    except FdtdError:
-                        break  # kernel not applicable to this grid
-                    eng.iterate(min(steps, 16))  # warm-up, graph instantiation
-                    eng.reset()
-                    eng.iterate(steps)
-                    ms, _ = eng.last_timing()
-                    tile = 0 if own else eng.stats()["tile_y"]
-                    eng.close()
-                    table.append(dict(kernel=k, tile_y=tile, stages=s, x_chunk=xc, ms_step=ms / steps))
-                    if verbose:
-                        print(f"kernel={k:5s} tile_y={tile} stages={s} x_chunk={xc:3d}  {ms / steps * 1e3:8.1f} us/step",
-                              flush=True)
+            for s in stages:
+                for xc in xchunks:
+                    if not candidate(k, ty, s, xc):
+                        break
     best = min(table, key=lambda r: r["ms_step"])
     return best, table
 
