@@ -125,3 +125,25 @@ def test_batched_jobs_hold_no_resident_buffers():
         assert (es[0].stats()["device_bytes"] > base) == (kernel == "auto")
         for e in (b0, b, *es):
             e.close()
+
+
+@pytest.mark.parametrize("n,bins", [((130, 128, 120), 0), ((33, 33, 33), 1)])
+def test_batch_after_an_asynchronous_iterate(n, bins):
+    """A batch takes jobs whose asynchronous steps were not waited for, on
+    whichever kernels it steps them."""
+    cop = CompressedOperator(Operator(_scene(n)))
+    jobs = 2 if bins == 0 else 16
+    es, ref = ([Engine(cop, max_timesteps=300, kernel="tma") for _ in range(jobs)] for _ in range(2))
+    b = Batch(es)
+    assert b.stats()["num_bins"] == bins
+    es[0].iterate_async(30)
+    b.iterate(20)
+    es[0].wait()
+    assert [e.num_timesteps for e in es[:2]] == [50, 20]
+    for e, steps in zip(ref, (50, 20)):
+        e.iterate(steps)
+    for e, r in zip(es[:2], ref):
+        for x, y in zip(e.fields(), r.fields()):
+            assert x.tobytes() == y.tobytes()
+    for e in (b, *es, *ref):
+        e.close()

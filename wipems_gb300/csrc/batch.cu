@@ -704,6 +704,9 @@ int fdtd_batch_iterate(fdtd_batch_t b, uint32_t n) {
     CK(cudaSetDevice(b->device));
     b->last_launches = 0;
     int rc;
+    // a job's own asynchronous steps come first; what they report stays in
+    // its error word and is returned below
+    for (fdtd_engine_s* e : b->own) fdtd_engine_wait(e);
     if (!b->bins.empty() && b->graph_steps > 1 && n >= b->graph_steps && (rc = batch_graph(b))) return rc;
     // what the jobs' own streams still hold (a reset, say) comes first
     for (fdtd_engine_s* e : b->jobs) {
