@@ -147,3 +147,14 @@ def test_batch_after_an_asynchronous_iterate(n, bins):
             assert x.tobytes() == y.tobytes()
     for e in (b, *es, *ref):
         e.close()
+
+
+def test_interval_graph_of_many_timesteps():
+    """A probe interval above 65536 timesteps replays its graph as a shorter
+    one does: one chunk's launches, one counter launch."""
+    cop = CompressedOperator(Operator(_scene((6, 5, 7))))
+    e = Engine(cop, max_timesteps=200000, probe_interval=70000, kernel="tma")
+    e.iterate(70000)
+    assert e.last_timing()[1] in (2 * 70000 + 1, 2 * 70000 + 2)  # and the sample of numTS 0
+    e.iterate(70000)
+    assert e.last_timing()[1] == 2 * 70000 + 1 and list(e.samples().ts) == [0, 70000, 140000]

@@ -1083,9 +1083,9 @@ int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
             left -= run;
             continue;
         }
-        // run to the next sample or frequency-domain step; the counter
-        // advances once per run
-        uint32_t run = std::min(left, 1u << 16);
+        // run to the next sample or frequency-domain step, an interval's graph
+        // however long it is; the counter advances once per run
+        uint32_t run = std::min(left, std::max(e->chunk ? e->interval : 0u, 1u << 16));
         if (e->interval) run = std::min(run, e->interval - e->ts % e->interval);
         if (fd_on) run = std::min(run, e->fd_interval - e->ts % e->fd_interval);
         if (e->chunk && run == e->interval) {
