@@ -1,5 +1,7 @@
 """Resident runs (the default kernel choice) against the kernels that read the
 fields of every timestep from memory: the same bits."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -158,3 +160,45 @@ def test_interval_graph_of_many_timesteps():
     assert e.last_timing()[1] in (2 * 70000 + 1, 2 * 70000 + 2)  # and the sample of numTS 0
     e.iterate(70000)
     assert e.last_timing()[1] == 2 * 70000 + 1 and list(e.samples().ts) == [0, 70000, 140000]
+
+
+def test_engines_that_share_the_gpu():
+    """Asynchronous calls run on the half-step kernels, which overlap; a
+    synchronous call runs resident while no other engine has timesteps in
+    flight.  Engines on their own streams and threads, resident or not, give
+    the bits of one that runs alone."""
+    walls = (BC_PEC, BC_PML, BC_MUR, BC_PEC)
+    sizes = ((22, 35, 40), (30, 28, 33), (33, 21, 30), (90, 88, 70))
+    cops = [CompressedOperator(Operator(_scene(n, w))) for n, w in zip(sizes, walls)]
+    ref = [Engine(c, max_timesteps=3000, kernel="tma") for c in cops]
+    es = [Engine(c, max_timesteps=3000) for c in cops]
+    for e in ref:
+        e.iterate(2200)
+    for e in es:
+        e.iterate_async(100)
+    for e in es:
+        e.wait()
+        assert e.last_timing()[1] > 200
+    es[0].iterate_async(50)
+    es[1].iterate(50)  # beside the first engine's
+    assert es[1].last_timing()[1] > 100
+    es[0].wait()
+    es[0].iterate(50)
+    assert es[0].last_timing()[1] <= 4
+    es[1].iterate(50)
+    for e in es[2:]:
+        e.iterate(100)
+        assert e.last_timing()[1] <= 4 * (1 + 100 // (64 * e.interval))
+    th = [threading.Thread(target=lambda e=e: [e.iterate(k) for k in (1, 499, 1500)]) for e in es]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for e, r in zip(es, ref):
+        assert e.num_timesteps == 2200
+        _same(e, r)
+    b = es[3]
+    b.iterate_async(10)
+    b.close()  # an engine that ends with timesteps in flight no longer counts
+    es[0].iterate(50)
+    assert es[0].last_timing()[1] <= 4

@@ -704,6 +704,8 @@ int fdtd_batch_iterate(fdtd_batch_t b, uint32_t n) {
     CK(cudaSetDevice(b->device));
     b->last_launches = 0;
     int rc;
+    InFlight flight;
+    flight.enter(b->device);
     // a job's own asynchronous steps come first; what they report stays in
     // its error word and is returned below
     for (fdtd_engine_s* e : b->own) fdtd_engine_wait(e);

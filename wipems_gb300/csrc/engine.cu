@@ -541,6 +541,7 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
     }
     CK(cudaEventCreate(&e->ev0));
     CK(cudaEventCreate(&e->ev1));
+    for (cudaEvent_t& ev : e->ev_run) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     e->TY = (opts && opts->tile_y > 0) ? opts->tile_y : 8;
     if (e->TY > 8 || e->TY < 1) {
         set_error("tile_y must be 1..8");
@@ -1030,65 +1031,35 @@ int fdtd_engine_add_probe(fdtd_engine_t e, const fdtd_probe_desc* p, uint32_t* s
     return FDTD_OK;
 }
 
-int fdtd_engine_iterate(fdtd_engine_t e, uint32_t n) {
-    const int rc = fdtd_engine_iterate_async(e, n);
-    if (rc) return rc;
-    return fdtd_engine_wait(e);
-}
-
-int fdtd_engine_wait(fdtd_engine_t e) {
-    if (!e) return FDTD_ERR_ARG;
-    if (!e->pending) return FDTD_OK;
-    CK(cudaSetDevice(e->device));
-    e->pending = false;
-    CK(cudaEventSynchronize(e->ev1));
-    float ms = 0;
-    CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
-    e->last_ms = ms;
-    return check_error_word(e);
-}
-
-int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
+// The checks and the start of an iterate call; n: the timesteps it may take.
+static int begin_steps(fdtd_engine_t e, uint32_t* n) {
     if (!e) return FDTD_ERR_ARG;
     if (e->pending) {
         set_error("fdtd_engine_iterate_async: the previous asynchronous iterate was not waited for");
         return FDTD_ERR_STATE;
     }
     if (e->end_crit > 0) {  // a stopped job stays stopped; never step past the timestep cap
-        if (e->done || e->ts >= e->stop_ts) n = 0;
-        else n = std::min(n, e->stop_ts - e->ts);
+        if (e->done || e->ts >= e->stop_ts) *n = 0;
+        else *n = std::min(*n, e->stop_ts - e->ts);
     }
     CK(cudaSetDevice(e->device));
     e->last_launches = 0;
-    int rc;
     CK(cudaEventRecord(e->ev0, e->stream));
-    if ((rc = start(e))) return rc;
+    return start(e);
+}
+
+// n timesteps on the half-step kernels
+static int queue_half_steps(fdtd_engine_t e, uint32_t n) {
     const bool fd_on = e->fd_interval && !e->h_freq.empty() && e->ps.nprobe;
-    if (e->resident && n > 0 && !e->res_ready) {
-        if ((rc = setup_resident(e))) return rc;
-        e->resident = e->res_ready;
-        if (!e->resident && e->interval && e->use_graphs && (rc = build_chunk_graph(e))) return rc;
-    }
-    uint32_t left = n;
-    while (left > 0) {
-        // A single timestep pays for a whole trip of the state into shared memory
-        // and back: without Mur or RLC launches beside the half-steps those are
-        // faster (us per call, resident / half-steps: 65^3 PEC 40 / 40, 91^3 49 /
-        // 46, 102^3 61 / 52, 65 x 71 x 61 dispersive 49 / 44; with Mur 51 x 42 x 61
-        // 41 / 56).  Two timesteps are faster resident on all of these.
-        if (e->resident && (left > 1 || e->mur.nface || e->rlc.count)) {
-            const uint32_t run = resident_run(e, left);
-            if ((rc = launch_resident(e, run, e->stream))) return rc;
-            e->ts += run;
-            left -= run;
-            continue;
-        }
+    int rc;
+    for (uint32_t left = n; left > 0;) {
         // run to the next sample or frequency-domain step, an interval's graph
         // however long it is; the counter advances once per run
-        uint32_t run = std::min(left, std::max(e->chunk ? e->interval : 0u, 1u << 16));
+        uint32_t run = std::min(left, std::max(e->use_graphs ? e->interval : 0u, 1u << 16));
         if (e->interval) run = std::min(run, e->interval - e->ts % e->interval);
         if (fd_on) run = std::min(run, e->fd_interval - e->ts % e->fd_interval);
-        if (e->chunk && run == e->interval) {
+        if (e->use_graphs && run == e->interval) {
+            if ((rc = build_chunk_graph(e))) return rc;
             CK(cudaGraphLaunch(e->chunk, e->stream));
             e->last_launches += e->chunk_launches;
         } else {
@@ -1100,8 +1071,84 @@ int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
         left -= run;
         if (fd_on && e->ts % e->fd_interval == 0 && (rc = launch_fd(e, e->ts))) return rc;
     }
+    return FDTD_OK;
+}
+
+// n timesteps, run by run: a resident run has the whole GPU, so it is chosen
+// while no other engine of the device has timesteps in flight, and looked at
+// again for each run (two runs are queued ahead).  Engines that share the GPU
+// overlap better on the half-step kernels (us per timestep of all, resident /
+// half-steps: 8 x 41^3 PEC 21.7 / 14.4, 4 x 91^3 38.6 / 29.3, 8 x 47 x 33 x 61
+// UPML 32.5 / 20.2).
+static int queue_steps(fdtd_engine_t e, uint32_t n) {
+    int rc;
+    if (e->resident && n > 0 && !e->res_ready) {
+        if ((rc = setup_resident(e))) return rc;
+        e->resident = e->res_ready;
+    }
+    if (!e->resident) return queue_half_steps(e, n);
+    uint32_t left = n;
+    for (uint32_t k = 0; left > 0; ++k) {
+        if (k >= 2) CK(cudaEventSynchronize(e->ev_run[k & 1]));
+        const uint32_t run = resident_run(e, left);
+        // A single timestep pays for a whole trip of the state into shared memory
+        // and back: without Mur or RLC launches beside the half-steps those are
+        // faster (us per call, resident / half-steps: 65^3 PEC 40 / 40, 91^3 49 /
+        // 46, 102^3 61 / 52, 65 x 71 x 61 dispersive 49 / 44; with Mur 51 x 42 x 61
+        // 41 / 56).  Two timesteps are faster resident on all of these.
+        if (InFlight::count(e->device) == 1 && (left > 1 || e->mur.nface || e->rlc.count)) {
+            if ((rc = launch_resident(e, run, e->stream))) return rc;
+            e->ts += run;
+        } else if ((rc = queue_half_steps(e, run))) {
+            return rc;
+        }
+        left -= run;
+        if (left) CK(cudaEventRecord(e->ev_run[k & 1], e->stream));
+    }
+    return FDTD_OK;
+}
+
+int fdtd_engine_iterate(fdtd_engine_t e, uint32_t n) {
+    int rc;
+    if ((rc = begin_steps(e, &n))) return rc;
+    e->flight.enter(e->device);
+    rc = queue_steps(e, n);
+    if (rc == FDTD_OK) {
+        const cudaError_t ce = cudaEventRecord(e->ev1, e->stream);
+        if (ce != cudaSuccess) {
+            set_error(std::string("cudaEventRecord: ") + cudaGetErrorString(ce));
+            rc = FDTD_ERR_CUDA;
+        }
+    }
+    if (rc) {
+        e->flight.leave();
+        return rc;
+    }
+    e->pending = true;
+    return fdtd_engine_wait(e);
+}
+
+int fdtd_engine_wait(fdtd_engine_t e) {
+    if (!e) return FDTD_ERR_ARG;
+    if (!e->pending) return FDTD_OK;
+    CK(cudaSetDevice(e->device));
+    e->pending = false;
+    const cudaError_t ce = cudaEventSynchronize(e->ev1);
+    e->flight.leave();
+    CK(ce);
+    float ms = 0;
+    CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+    e->last_ms = ms;
+    return check_error_word(e);
+}
+
+// Engines stepped this way share the GPU: the half-step kernels.
+int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
+    int rc;
+    if ((rc = begin_steps(e, &n)) || (rc = queue_half_steps(e, n))) return rc;
     CK(cudaEventRecord(e->ev1, e->stream));
     e->pending = true;
+    e->flight.enter(e->device);
     return FDTD_OK;
 }
 

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -26,6 +27,29 @@ namespace wipems {
             return FDTD_ERR_CUDA;                                          \
         }                                                                  \
     } while (0)
+
+// How many engines and batches of this process have timesteps in flight on a
+// device; one that has them enters, and leaves when they are done or it ends.
+class InFlight {
+    static std::atomic<int>& at(int device) {
+        static std::atomic<int> n[64];
+        return n[device & 63];
+    }
+    int device = -1;
+
+  public:
+    static int count(int device) { return at(device).load(std::memory_order_relaxed); }
+    void enter(int dev) {
+        leave();
+        device = dev;
+        at(dev).fetch_add(1, std::memory_order_relaxed);
+    }
+    void leave() {
+        if (device >= 0) at(device).fetch_sub(1, std::memory_order_relaxed);
+        device = -1;
+    }
+    ~InFlight() { leave(); }
+};
 
 struct DevHalfBufs {
     DevBuf<uint8_t> idx;
@@ -119,6 +143,7 @@ struct fdtd_engine_s {
     bool energy_on_probe = true;
     bool use_graphs = true;
     bool pending = false;    // an asynchronous iterate was launched, not yet waited for
+    InFlight flight;
     double end_crit = 0;     // > 0: stop on the device (energy decay or stop_ts)
     uint32_t stop_ts = 0;
     bool done = false;       // as of the last control-word read
@@ -160,10 +185,13 @@ struct fdtd_engine_s {
     cudaGraphExec_t chunk = nullptr;
     uint64_t chunk_launches = 0;  // kernels in it
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_run[2] = {nullptr, nullptr};  // the last two runs of a call (queue_steps)
     double last_ms = 0;
     uint64_t last_launches = 0;
 
     ~fdtd_engine_s() {
+        for (cudaEvent_t ev : ev_run)
+            if (ev) cudaEventDestroy(ev);
         if (chunk) cudaGraphExecDestroy(chunk);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
