@@ -202,3 +202,16 @@ def test_engines_that_share_the_gpu():
     b.close()  # an engine that ends with timesteps in flight no longer counts
     es[0].iterate(50)
     assert es[0].last_timing()[1] <= 4
+
+
+@pytest.mark.parametrize("n", [(20, 21, 22), (33, 30, 34), (22, 37, 65)])
+def test_one_plane_chunks(n):
+    """The current kernel with fewer registers for chunks of one plane (UPML,
+    16-bit indices), on sample steps and between."""
+    cop = CompressedOperator(Operator(_scene(n, BC_PML)))
+    es = [Engine(cop, max_timesteps=300, kernel="tma", x_chunk=1), Engine(cop, max_timesteps=300, kernel="direct")]
+    for e in es:
+        e.iterate(37)
+        e.iterate(120)
+    assert es[0].stats()["x_chunk"] == 1
+    _same(*es)

@@ -483,8 +483,10 @@ __global__ void __launch_bounds__(TY * 32) k_volt_tma(const DevGrid g, const __g
                                    *g.d_ts + ts_off);
 }
 
-template <typename IdxT, int FEAT, bool GEO, bool ENERGY, int TY>
-__global__ void __launch_bounds__(TY * 32) k_curr_tma(const DevGrid g, const __grid_constant__ TmaMaps m,
+// MINB: blocks an SM should hold at once (1: as many registers as the compiler
+// likes), for chunks of one plane (see launch_curr_tma).
+template <typename IdxT, int FEAT, bool GEO, bool ENERGY, int TY, int MINB = 1>
+__global__ void __launch_bounds__(TY * 32, MINB) k_curr_tma(const DevGrid g, const __grid_constant__ TmaMaps m,
                                                       const TileInfo ti, int ts_off, int XC, int STAGES) {
     using L = StageLayout<IdxT, (FEAT & FEAT_UPML) != 0, false, TY>;
     extern __shared__ __align__(128) float smem_raw[];

@@ -19,11 +19,27 @@ void launch_volt_tma(fdtd_engine_s* e, int ts_off) {
                                                                            e->stages);
 }
 
+// Current kernels with a variant of 40 registers, so that an SM holds 12 blocks
+// instead of 10.  Blocks of one plane (small grids) wait for it all their life,
+// and more of them hide that: UPML 56^3 lines 11.4 -> 10.7 us per timestep, 8
+// such engines at once 57.3 -> 46.2, 61^3 69.0 -> 61.6.  Longer chunks prefer
+// the registers (101^3 26.7 -> 29.8, 257^3 249 -> 255).  The other feature sets
+// need 32 registers anyway or more than 48.
+template <typename IdxT, int FEAT, bool GEO, int TY>
+constexpr bool kOnePlaneBlocks = sizeof(IdxT) == 2 && FEAT == FEAT_UPML && !GEO && TY == TMA_TY;
+
 template <typename IdxT, int FEAT, bool GEO, bool EN, int TY>
 void launch_curr_tma(fdtd_engine_s* e, int ts_off) {
     constexpr bool UP = (FEAT & FEAT_UPML) != 0;
     const size_t sm = StageLayout<IdxT, UP, false, TY>::smem(e->stages);
     dim3 grid((e->N[2] - 1 + 31) / 32, (e->N[1] - 1 + TY - 1) / TY, (e->N[0] - 1 + e->XC - 1) / e->XC);
+    if constexpr (kOnePlaneBlocks<IdxT, FEAT, GEO, TY>) {
+        if (e->XC == 1) {
+            k_curr_tma<IdxT, FEAT, GEO, EN, TY, 12><<<grid, dim3(32, TY), sm, e->stream>>>(e->g, e->maps, e->ti, ts_off,
+                                                                                           e->XC, e->stages);
+            return;
+        }
+    }
     k_curr_tma<IdxT, FEAT, GEO, EN, TY><<<grid, dim3(32, TY), sm, e->stream>>>(e->g, e->maps, e->ti, ts_off, e->XC,
                                                                                e->stages);
 }
@@ -61,6 +77,11 @@ cudaError_t smem_attr_one(int bytes) {
                         cudaFuncSetAttribute(k_curr_tma<IdxT, FEAT, GEO, false, 8>, a, bytes)};
     for (cudaError_t x : r)
         if (x != cudaSuccess) return x;
+    if constexpr (kOnePlaneBlocks<IdxT, FEAT, GEO, TMA_TY>) {
+        for (const void* k : {(const void*)k_curr_tma<IdxT, FEAT, GEO, true, TMA_TY, 12>,
+                              (const void*)k_curr_tma<IdxT, FEAT, GEO, false, TMA_TY, 12>})
+            if (const cudaError_t x = cudaFuncSetAttribute(k, a, bytes)) return x;
+    }
     return cudaSuccess;
 }
 
