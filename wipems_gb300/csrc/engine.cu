@@ -244,8 +244,8 @@ int upload_probes(fdtd_engine_s* e) {
     return FDTD_OK;
 }
 
-int build_chunk_graph(fdtd_engine_s* e) {
-    if (e->chunk) return FDTD_OK;
+int build_chunk_graph(fdtd_engine_s* e, cudaGraphExec_t* chunk) {
+    if (*chunk) return FDTD_OK;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     int rc;
@@ -263,10 +263,10 @@ int build_chunk_graph(fdtd_engine_s* e) {
         set_error(std::string("cudaStreamEndCapture: ") + cudaGetErrorString(ce));
         return FDTD_ERR_CUDA;
     }
-    ce = cudaGraphInstantiate(&e->chunk, graph, 0);
+    ce = cudaGraphInstantiate(chunk, graph, 0);
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) {
-        e->chunk = nullptr;
+        *chunk = nullptr;
         set_error(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ce));
         return FDTD_ERR_CUDA;
     }
@@ -282,7 +282,6 @@ int start(fdtd_engine_s* e) {
             if ((rc = plan_resident(e))) return rc;
             e->resident = e->res_fits;
         }
-        if (e->interval && e->use_graphs && !e->resident && (rc = build_chunk_graph(e))) return rc;
     }
     if (e->need_initial_sample) {
         e->need_initial_sample = false;
@@ -586,8 +585,13 @@ int upload_engine(const fdtd_cop_s* c, const fdtd_engine_opts* opts, fdtd_engine
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
         // about 1280 resident threads per SM (5 blocks of 32 x 8, 10 of 32 x 4)
-        e->XC = auto_x_chunk({e->N}, (uint64_t)(1280 / (32 * e->tma_ty)) * (uint64_t)sms, TMA_TY,
-                             !e->use_tma || e->fused ? 16 : c->E.adex_orders || c->H.adex_orders ? 2 : 6);
+        const uint64_t blocks = (uint64_t)(1280 / (32 * e->tma_ty)) * (uint64_t)sms;
+        e->XC_shared = auto_x_chunk({e->N}, blocks);
+        e->XC_alone = auto_x_chunk({e->N}, blocks, TMA_TY,
+                                   !e->use_tma || e->fused ? 16 : c->E.adex_orders || c->H.adex_orders ? 2 : 6);
+        e->XC = e->XC_alone;
+    } else {
+        e->XC_alone = e->XC_shared = e->XC;
     }
     e->comp = c->comp;
     e->geo_on = c->geo;
@@ -1048,8 +1052,11 @@ static int begin_steps(fdtd_engine_t e, uint32_t* n) {
     return start(e);
 }
 
-// n timesteps on the half-step kernels
+// n timesteps on the half-step kernels (the engine is in flight)
 static int queue_half_steps(fdtd_engine_t e, uint32_t n) {
+    const bool shared = InFlight::count(e->device) > 1;
+    e->XC = shared ? e->XC_shared : e->XC_alone;
+    cudaGraphExec_t* chunk = &e->chunk[e->XC != e->XC_alone];
     const bool fd_on = e->fd_interval && !e->h_freq.empty() && e->ps.nprobe;
     int rc;
     for (uint32_t left = n; left > 0;) {
@@ -1059,8 +1066,8 @@ static int queue_half_steps(fdtd_engine_t e, uint32_t n) {
         if (e->interval) run = std::min(run, e->interval - e->ts % e->interval);
         if (fd_on) run = std::min(run, e->fd_interval - e->ts % e->fd_interval);
         if (e->use_graphs && run == e->interval) {
-            if ((rc = build_chunk_graph(e))) return rc;
-            CK(cudaGraphLaunch(e->chunk, e->stream));
+            if ((rc = build_chunk_graph(e, chunk))) return rc;
+            CK(cudaGraphLaunch(*chunk, e->stream));
             e->last_launches += e->chunk_launches;
         } else {
             const bool sample = e->interval && (e->ts + run) % e->interval == 0;
@@ -1108,11 +1115,12 @@ static int queue_steps(fdtd_engine_t e, uint32_t n) {
     return FDTD_OK;
 }
 
-int fdtd_engine_iterate(fdtd_engine_t e, uint32_t n) {
+// An iterate call up to its wait.
+static int queue_call(fdtd_engine_t e, uint32_t n, int (*queue)(fdtd_engine_t, uint32_t)) {
     int rc;
     if ((rc = begin_steps(e, &n))) return rc;
     e->flight.enter(e->device);
-    rc = queue_steps(e, n);
+    rc = queue(e, n);
     if (rc == FDTD_OK) {
         const cudaError_t ce = cudaEventRecord(e->ev1, e->stream);
         if (ce != cudaSuccess) {
@@ -1120,12 +1128,14 @@ int fdtd_engine_iterate(fdtd_engine_t e, uint32_t n) {
             rc = FDTD_ERR_CUDA;
         }
     }
-    if (rc) {
-        e->flight.leave();
-        return rc;
-    }
-    e->pending = true;
-    return fdtd_engine_wait(e);
+    e->pending = rc == FDTD_OK;
+    if (rc) e->flight.leave();
+    return rc;
+}
+
+int fdtd_engine_iterate(fdtd_engine_t e, uint32_t n) {
+    const int rc = queue_call(e, n, queue_steps);
+    return rc ? rc : fdtd_engine_wait(e);
 }
 
 int fdtd_engine_wait(fdtd_engine_t e) {
@@ -1144,12 +1154,7 @@ int fdtd_engine_wait(fdtd_engine_t e) {
 
 // Engines stepped this way share the GPU: the half-step kernels.
 int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
-    int rc;
-    if ((rc = begin_steps(e, &n)) || (rc = queue_half_steps(e, n))) return rc;
-    CK(cudaEventRecord(e->ev1, e->stream));
-    e->pending = true;
-    e->flight.enter(e->device);
-    return FDTD_OK;
+    return queue_call(e, n, queue_half_steps);
 }
 
 int fdtd_engine_set_fd(fdtd_engine_t e, const double* freqs, uint32_t nfreq, uint32_t fd_interval) {
@@ -1700,7 +1705,7 @@ int fdtd_engine_get_stats(fdtd_engine_t e, fdtd_engine_stats* st) {
     st->padded_nz = (uint32_t)e->Nzp;
     st->device_bytes = e->device_bytes;
     st->tile_y = (uint32_t)(e->fused ? FU_TY : (e->use_tma ? e->tma_ty : e->TY));
-    st->x_chunk = (uint32_t)e->XC;
+    st->x_chunk = (uint32_t)e->XC_alone;
     st->kernel = e->fused ? 2u : (e->use_tma ? 3u : 1u);
     return FDTD_OK;
 }

@@ -157,7 +157,8 @@ struct fdtd_engine_s {
     bool geo_on = false;
     int TY = 8;       // direct kernels: tile rows
     int tma_ty = 4;   // two-pass TMA kernels: tile rows (4 or 8)
-    int XC = 8;
+    int XC = 8;                    // x-chunk of the launches: one of
+    int XC_alone = 8, XC_shared = 8;  // alone on the GPU, beside other engines
     bool use_tma = true;
     bool fused = false;      // single-pass kernel, double-buffered fields
     FusedMaps fmaps{};
@@ -182,8 +183,8 @@ struct fdtd_engine_s {
     size_t smem_direct = 0;
     uint32_t num_tuples_e = 0, num_tuples_h = 0, upml_nodes = 0, ade_nodes = 0;
     uint64_t device_bytes = 0;
-    cudaGraphExec_t chunk = nullptr;
-    uint64_t chunk_launches = 0;  // kernels in it
+    cudaGraphExec_t chunk[2] = {nullptr, nullptr};  // a probe interval on the half-step kernels: XC_alone, XC_shared
+    uint64_t chunk_launches = 0;  // kernels in one
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t ev_run[2] = {nullptr, nullptr};  // the last two runs of a call (queue_steps)
     double last_ms = 0;
@@ -192,7 +193,8 @@ struct fdtd_engine_s {
     ~fdtd_engine_s() {
         for (cudaEvent_t ev : ev_run)
             if (ev) cudaEventDestroy(ev);
-        if (chunk) cudaGraphExecDestroy(chunk);
+        for (cudaGraphExec_t c : chunk)
+            if (c) cudaGraphExecDestroy(c);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
     }
@@ -205,12 +207,13 @@ namespace wipems {
 // plane each), blocks run in waves of `resident`, so the step costs
 // ceil(blocks / resident) * (2 + x_chunk); a chunk that leaves SMs idle in the
 // only wave is skipped, ties go to the longer chunk (fewer halo-plane
-// re-reads).  lines: the jobs' (Nx, Ny, Nz) triples.  longest <= 6: one job on
-// the half-step kernels, whose chunks are 1, 2 or 4 planes, or 6 with eight
-// waves to spare: longer ones end the voltage half-step far from where the
+// re-reads).  lines: the jobs' (Nx, Ny, Nz) triples.  longest <= 6: one job
+// alone on the GPU on the half-step kernels, whose chunks are 1, 2 or 4 planes,
+// or 6 with eight waves to spare: longer ones end the voltage half-step far from where the
 // current one starts, and what it left in L2 is gone (257^3 UPML 16 planes
 // 266 us per step, 8: 261, 6: 256, 4: 260; 161^3 UPML 8: 88, 6: 83, 4: 81.6;
-// 257^3 PEC 16: 202, 6 and 4: 194).  Otherwise 1, 2, 4, 8 or 16.  With
+// 257^3 PEC 16: 202, 6 and 4: 194; with other engines beside it that is so
+// anyway, and 8 x 161^3 PEC take 426 us with 4 planes, 394 with 8).  Otherwise 1, 2, 4, 8 or 16.  With
 // dispersion orders above 1 at most 2: the blocks inside such materials take
 // several times as long as the others (106 x 101 x 96 lines 4 planes 35.0 us
 // per step, 2: 31.5).
