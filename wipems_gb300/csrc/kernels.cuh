@@ -535,6 +535,18 @@ __device__ __forceinline__ float rlc_edge(const RlcSet& rs, uint32_t k, int numT
     return vd;
 }
 
+// A face's b with the node's own excitation, if any.
+__device__ __forceinline__ float mur_excite(const DevGrid& g, const MurSet& ms, int numTS, int c, long long o, float v) {
+    if (!ms.exc) return v;
+    const uint32_t t = ms.idx16 ? load_idx<uint16_t>(g.e.idx, o) : load_idx<uint32_t>(g.e.idx, o);
+    if (__float_as_uint(__ldg(&g.e.main[TAB_MAIN * t + 1]).z) & TF_EXC) {
+        float f[3] = {v, v, v};
+        excite_node<false>(g, f, t, numTS);
+        v = c == 0 ? f[0] : c == 1 ? f[1] : f[2];
+    }
+    return v;
+}
+
 // Component c of node p after the Mur passes of numTS: the b of the first
 // active face that writes it, with the node's excitation, else V.
 __device__ __forceinline__ float mur_final(const DevGrid& g, const MurSet& ms, int numTS, const int p[3], int c,
@@ -544,15 +556,7 @@ __device__ __forceinline__ float mur_final(const DevGrid& g, const MurSet& ms, i
         if (numTS < G.start_ts || c == G.ny || p[G.ny] != G.line) continue;
         const int nP = (G.ny + 1) % 3, nPP = (G.ny + 2) % 3;
         const long long loc = (long long)p[nP] * G.n1 + p[nPP];
-        float v = G.b[numTS & 1][(c == nP ? 0 : (long long)G.n0 * G.n1) + loc];
-        if (!ms.exc) return v;
-        const uint32_t t = ms.idx16 ? load_idx<uint16_t>(g.e.idx, o) : load_idx<uint32_t>(g.e.idx, o);
-        if (__float_as_uint(__ldg(&g.e.main[TAB_MAIN * t + 1]).z) & TF_EXC) {
-            float f[3] = {v, v, v};
-            excite_node<false>(g, f, t, numTS);
-            v = c == 0 ? f[0] : c == 1 ? f[1] : f[2];
-        }
-        return v;
+        return mur_excite(g, ms, numTS, c, o, G.b[numTS & 1][(c == nP ? 0 : (long long)G.n0 * G.n1) + loc]);
     }
     return g.V[c * g.comp + o];
 }
@@ -604,13 +608,13 @@ static __global__ void k_mur(const DevGrid g, const MurSet ms, const RlcSet rs, 
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int c = comps[q];
-                fin[q] = mur_final(g, ms, numTS, pos, c, ol);
                 bool mine = numTS >= F.start_ts;  // an earlier active face sharing this component writes it
                 for (int e = 0; e < fi; ++e) {
                     const MurDev& G = ms.f[e];
                     if (numTS >= G.start_ts && pos[G.ny] == G.line && c != G.ny) mine = false;
                 }
-                if (mine) V[c * C + ol] = fin[q];
+                if (mine) V[c * C + ol] = fin[q] = mur_excite(g, ms, numTS, c, ol, b[q * n + loc]);
+                else if (next) fin[q] = mur_final(g, ms, numTS, pos, c, ol);
             }
             if (next && numTS + 1 >= F.start_ts) {
                 float* d = F.b[(numTS & 1) ^ 1];
