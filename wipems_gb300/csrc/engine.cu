@@ -1458,6 +1458,7 @@ int fdtd_engine_energy(fdtd_engine_t e, double* energy) {
 
 // The fields without device scratch: rows to the host as they are, axes turned
 // over there.
+constexpr size_t kDirectBytes = (size_t)256 << 10;
 static int get_fields_host(fdtd_engine_t e, float* volt, float* curr) {
     const size_t n = (size_t)e->N[0] * e->N[1] * e->N[2];
     const std::unique_ptr<float[]> tmp(e->rot ? new (std::nothrow) float[n] : nullptr);
@@ -1494,12 +1495,10 @@ int fdtd_engine_get_fields(fdtd_engine_t e, float* volt, float* curr) {
     const size_t plane = (size_t)M[1] * M[2];
     // small arrays in the operator's axes: the copies alone (26 x 11 x 32
     // lines 28 us, packed first 39; 41^3 lines 70 us, packed 49)
-    if (e->rot == 0 && 3 * M[0] * plane * sizeof(float) < kFreshBytes) return get_fields_host(e, volt, curr);
+    if (e->rot == 0 && 3 * M[0] * plane * sizeof(float) < kDirectBytes) return get_fields_host(e, volt, curr);
     // planes of the first axis, of all components, through a packed array, or
     // turned over on the host where the device has no memory for one
-    DevBuf<float> once;
-    float* scratch = nullptr;
-    const uint32_t planes = 3 * M[0], slab = readback_planes(planes, plane, e->dump, once, e->device_bytes, e->stream, &scratch);
+    const uint32_t planes = 3 * M[0], slab = readback_planes(planes, plane, e->dump, e->device_bytes, e->stream);
     if (!slab) return get_fields_host(e, volt, curr);
     int rc;
     const int f = (2 + e->rot) % 3;
@@ -1511,10 +1510,10 @@ int fdtd_engine_get_fields(fdtd_engine_t e, float* volt, float* curr) {
             const uint32_t hi = std::min(planes, lo + slab);
             const dim3 grid((M[2] + 31) / 32, ((f == 0 ? hi - lo : M[1]) + 31) / 32,
                             std::min(f == 0 ? M[1] : hi - lo, 65535u));
-            k_pack_field<<<grid, 256, 0, e->stream>>>(which ? e->cur_I() : e->cur_V(), scratch, (int)M[0], (int)M[1],
+            k_pack_field<<<grid, 256, 0, e->stream>>>(which ? e->cur_I() : e->cur_V(), e->dump.p, (int)M[0], (int)M[1],
                                                       (int)M[2], e->comp, e->g.sx, e->Nzp, e->rot, (int)lo, (int)hi);
             if ((rc = check_launch())) return rc;
-            CK(cudaMemcpyAsync(dst + lo * plane, scratch, (hi - lo) * plane * sizeof(float), cudaMemcpyDeviceToHost,
+            CK(cudaMemcpyAsync(dst + lo * plane, e->dump.p, (hi - lo) * plane * sizeof(float), cudaMemcpyDeviceToHost,
                                e->stream));
         }
     }

@@ -12,34 +12,34 @@
 
 namespace wipems {
 
-constexpr size_t kFreshBytes = (size_t)256 << 10;  // allocators give arrays above this fresh pages
-
-// Whether the pages of a host array are there already, by a sample of them
-// (a system call of 0.4 us each): an array that was written before, or memory
-// that the allocator hands out again.
+// Whether the pages of a host array are there already, by a sample of them: an
+// array that was written before, or memory that the allocator hands out again.
 inline bool pages_mapped(const void* p, size_t bytes) {
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    const int n = bytes < (size_t)4 << 20 ? 4 : 16;
-    for (int k = 0; k < n; ++k) {
-        const uintptr_t a = (uintptr_t)p + (bytes - 1) / (n - 1) * k;
+    for (size_t k = 0; k < 16; ++k) {
+        const uintptr_t a = (uintptr_t)p + (bytes - 1) / 15 * k;
         unsigned char there = 0;
         if (mincore((void*)(a / page * page), page, &there) != 0 || !(there & 1)) return false;
     }
     return true;
 }
 
-// Maps the pages of a large host destination before the device writes to it,
-// a share per thread.  A fresh array's pages do not exist yet, and faulting
-// them in one by one under the copy takes many times the copy: both fields of
-// 257^3 lines (408 MB) took 335 ms to read, 6.4 ms with their pages mapped by
-// 16 threads first.  Small arrays are touched by the calling thread alone, and
-// mapped ones are left alone (touching those took 1.1 ms of the 4.1 ms that
-// the same fields took into arrays written before).
+// Writes to every page of a large host destination before the device does, a
+// share per thread.  A fresh array's pages do not exist yet, and faulting them
+// in one by one under the copy takes many times the copy: both fields of 257^3
+// lines (408 MB) took 335 ms to read, 6.4 ms with their pages mapped by 16
+// threads first.  Pages that are mapped are touched all the same: where they
+// come from memory that the program used for something else before, a copy
+// into them took up to ten times as long without (193^3 lines 34 ms, 1.4
+// touched).  That is quick, so fewer threads do it.  Under 4 MB it costs more
+// than it saves (a dump of 0.8 MB 55 us, touched 63).  The contents are lost
+// either way: the whole array is the destination.
 inline void touch_pages(void* p, size_t bytes) noexcept {
-    if (bytes < kFreshBytes || pages_mapped(p, bytes)) return;
-    const size_t page = 4096;
+    if (bytes < (size_t)4 << 20) return;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned nt = (unsigned)std::max<size_t>(1, std::min<size_t>(std::min(hw, 16u), bytes >> 21));
+    const unsigned nt = (unsigned)std::max<size_t>(
+        1, std::min<size_t>(std::min(hw, 16u), pages_mapped(p, bytes) ? bytes >> 26 : bytes >> 21));
     auto part = [=](unsigned k) {
         volatile char* b = static_cast<volatile char*>(p);
         const size_t lo = bytes / nt * k, hi = k + 1 == nt ? bytes : bytes / nt * (k + 1);
@@ -56,23 +56,17 @@ inline void touch_pages(void* p, size_t bytes) noexcept {
         if (t.joinable()) t.join();
 }
 
-constexpr size_t kReadbackFloats = (size_t)32 << 20;  // scratch of a readback, at most (128 MB), and
-constexpr size_t kReadbackKept = (size_t)4 << 20;     // what of it an engine keeps for the next one (16 MB)
+constexpr size_t kReadbackFloats = (size_t)4 << 20;  // scratch of a readback (16 MB; a plane if that is more)
 
 // Planes (of `plane` floats each, at most `planes`) that a readback packs at
-// a time, with a scratch for them: `keep` if that is small, else `once`, which
-// the caller gives back.  Where memory is short fewer planes at a time, down
-// to one; 0 if there is not even that.
-inline uint32_t readback_planes(uint32_t planes, size_t plane, DevBuf<float>& keep, DevBuf<float>& once,
-                                uint64_t& kept_bytes, cudaStream_t st, float** scratch) {
-    uint64_t bytes = 0;  // of `once`: not the engine's
-    for (uint32_t n = (uint32_t)std::min<size_t>(planes, std::max<size_t>(1, kReadbackFloats / plane)); n > 0; n /= 2) {
-        const bool small = n * plane <= std::max(kReadbackKept, keep.n);
-        if ((small ? keep.grow(n * plane, kept_bytes, st) : once.grow(n * plane, bytes, st)) != FDTD_OK) continue;
-        *scratch = small ? keep.p : once.p;
-        return n;
-    }
-    return 0;
+// a time, in a scratch that the engine keeps (a larger one, allocated and
+// freed by each call, took up to 100 ms where the memory pool had to grow).
+// Where memory is short fewer planes at a time, down to one; 0 if there is not
+// even that.
+inline uint32_t readback_planes(uint32_t planes, size_t plane, DevBuf<float>& scratch, uint64_t& bytes, cudaStream_t st) {
+    uint32_t n = (uint32_t)std::min<size_t>(planes, std::max<size_t>(1, std::max(kReadbackFloats, scratch.n) / plane));
+    while (n > 0 && scratch.grow(n * plane, bytes, st) != FDTD_OK) n /= 2;
+    return n;
 }
 
 // One component from device axes to the operator's (device axis a = operator
