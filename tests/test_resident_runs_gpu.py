@@ -8,6 +8,8 @@ import pytest
 from wipems_gb300 import Batch, CompressedOperator, Engine, Operator, Scene
 from wipems_gb300.fdtd import BC_MUR, BC_PEC, BC_PMC, BC_PML
 
+from test_random_gpu import EXT_SEEDS, GRADED_SEEDS, NR_TS, SEEDS, _splits, random_scene, random_scene_ext
+
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("libs")]
 
 
@@ -215,3 +217,64 @@ def test_one_plane_chunks(n):
         e.iterate(120)
     assert es[0].stats()["x_chunk"] == 1
     _same(*es)
+
+
+@pytest.mark.parametrize("interval,fd,runs", [(0, 0, 3), (3, 0, 11), (7, 0, 5), (3, 1, 11), (0, 1, 9), (11, 5, 3)])
+def test_run_splits(interval, fd, runs):
+    """One call over the limits of a run: 1024 timesteps, 64 samples and 256
+    frequency-domain steps."""
+    cop = CompressedOperator(Operator(_scene((22, 25, 30))))
+    es = [Engine(cop, max_timesteps=3000, probe_interval=interval, kernel=k) for k in ("auto", "tma")]
+    for e in es:
+        if fd:
+            e.set_frequencies(np.linspace(5e9, 30e9, 3), fd_interval=fd)
+        e.iterate(2100)
+    per_run = 2 + (interval > 0) + (fd > 0)  # the run, its samples, energies and frequency-domain sums
+    initial = (interval > 0) + (fd > 0)      # of numTS 0
+    n = es[0].last_timing()[1] - initial
+    assert 2 * runs <= n <= per_run * runs, n
+    _same(*es)
+    if fd:
+        assert es[0].fd_results()[0].tobytes() == es[1].fd_results()[0].tobytes()
+        assert es[0].fd_results()[1] == 2100 // fd + 1
+
+
+@pytest.mark.parametrize("n,wall,fits", [((104, 100, 98), BC_PEC, True), ((112, 111, 110), BC_PEC, False),
+                                         ((80, 80, 80), BC_PML, True), ((92, 90, 88), BC_PML, False),
+                                         ((90, 88, 70), BC_MUR, True), ((104, 101, 99), BC_MUR, False)])
+def test_grids_around_the_capacity(n, wall, fits):
+    cop = CompressedOperator(Operator(_scene(n, wall)))
+    es = [Engine(cop, max_timesteps=300, kernel=k) for k in ("auto", "tma")]
+    for e in es:
+        e.iterate(40)
+    assert (es[0].last_timing()[1] <= 5) == fits
+    assert es[1].last_timing()[1] > 80
+    _same(*es)
+
+
+def test_batch_of_resident_jobs():
+    cop = CompressedOperator(Operator(_scene((61, 60, 62), BC_PML)))
+    es = [Engine(cop, max_timesteps=300, kernel="tma") for _ in range(3)]
+    b = Batch(es, x_chunk=64, blocks_per_sm=-1, chains=2)
+    assert b.stats()["num_bins"] == 0  # nothing left for the batched kernels
+    b.iterate(50)
+    assert b.stats()["last_launches"] <= 3 * 3
+
+
+@pytest.mark.parametrize("seed", SEEDS + GRADED_SEEDS + EXT_SEEDS)
+def test_random_scenes_on_the_default_engine(seed):
+    """The random sweeps with the engine's own choice of kernels, resident
+    where the scene allows, in split runs."""
+    ext = seed in EXT_SEEDS
+    op = Operator(random_scene_ext(seed) if ext else random_scene(seed, graded=seed in GRADED_SEEDS))
+    cop = CompressedOperator(op)
+    ref = Engine(cop, kernel="direct")
+    ref.iterate(NR_TS)
+    eng = Engine(cop)
+    rng = np.random.default_rng(4000 + seed)
+    for k in _splits(rng, NR_TS):
+        eng.iterate(k)
+    _same(eng, ref)
+    for p in op.probes:
+        if p.enabled and p.type in (0, 1):
+            assert eng.probe_now(p) == ref.probe_now(p)
