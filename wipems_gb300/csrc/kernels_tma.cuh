@@ -484,13 +484,10 @@ __global__ void __launch_bounds__(TY * 32) k_volt_tma(const DevGrid g, const __g
 }
 
 // MINB: blocks an SM should hold at once (1: as many registers as the compiler
-// likes), for chunks of one plane (see launch_curr_tma).  With dispersion
-// orders above 1, 64 registers as in the voltage kernel: the compiler takes up
-// to 90 for their states, and 5 blocks per SM (91^3 lines 31.1 us per timestep,
-// 8 such engines at once 206; with 8 blocks 29.6 and 185).
+// likes), for chunks of one plane (see launch_curr_tma).
 template <typename IdxT, int FEAT, bool GEO, bool ENERGY, int TY, int MINB = 1>
-__global__ void __launch_bounds__(TY * 32, (FEAT & FEAT_ADEX) ? 1024 / (32 * TY) : MINB)
-    k_curr_tma(const DevGrid g, const __grid_constant__ TmaMaps m, const TileInfo ti, int ts_off, int XC, int STAGES) {
+__global__ void __launch_bounds__(TY * 32, MINB) k_curr_tma(const DevGrid g, const __grid_constant__ TmaMaps m,
+                                                      const TileInfo ti, int ts_off, int XC, int STAGES) {
     using L = StageLayout<IdxT, (FEAT & FEAT_UPML) != 0, false, TY>;
     extern __shared__ __align__(128) float smem_raw[];
     float* smem = aligned_smem(smem_raw);
