@@ -441,12 +441,12 @@ typedef struct {
                                  size by a wave model) */
     int      kernel;          /* 0 = default: with no tiling given (tile_y,
                                      x_chunk, stages 0) and no end criterion,
-                                     fdtd_engine_iterate runs a grid that fits
-                                     in the GPU's shared memory resident while
-                                     no other engine of the process has
-                                     timesteps in flight on the device;
-                                     otherwise, and in
-                                     fdtd_engine_iterate_async, the
+                                     a grid that fits in the GPU's shared
+                                     memory runs resident while no other engine
+                                     of the process has timesteps in flight on
+                                     the device (asynchronous calls: from the
+                                     second one that is alone on), or among
+                                     many where that is faster; otherwise the
                                      TMA-pipelined two-pass kernels (3).
                                      Either way the same bits,
                                  1 = direct-load kernels,

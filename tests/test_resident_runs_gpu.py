@@ -170,7 +170,7 @@ def test_engines_that_share_the_gpu():
     flight.  Engines on their own streams and threads, resident or not, give
     the bits of one that runs alone."""
     walls = (BC_PEC, BC_PML, BC_MUR, BC_PEC)
-    sizes = ((22, 35, 40), (30, 28, 33), (33, 21, 30), (90, 88, 70))
+    sizes = ((42, 35, 40), (46, 33, 61), (45, 40, 44), (90, 88, 70))
     cops = [CompressedOperator(Operator(_scene(n, w))) for n, w in zip(sizes, walls)]
     ref = [Engine(c, max_timesteps=3000, kernel="tma") for c in cops]
     es = [Engine(c, max_timesteps=3000) for c in cops]
@@ -204,6 +204,30 @@ def test_engines_that_share_the_gpu():
     b.close()  # an engine that ends with timesteps in flight no longer counts
     es[0].iterate(50)
     assert es[0].last_timing()[1] <= 4
+    for launches in (100, 0):  # an asynchronous call counts as alone after one that was
+        es[0].iterate_async(50)
+        es[0].wait()
+        assert (es[0].last_timing()[1] > 100) == bool(launches)
+    ref[0].iterate(150)
+    _same(es[0], ref[0])
+
+
+def test_many_engines_with_upml():
+    """Engines that join a crowd of four or more run resident where that is the
+    faster way for many, with the same bits."""
+    cop = CompressedOperator(Operator(_scene((61, 60, 62), BC_PML)))
+    es = [Engine(cop, max_timesteps=300) for _ in range(7)]
+    ref = Engine(cop, max_timesteps=300, kernel="tma")
+    ref.iterate(150)
+    for steps in (100, 50):
+        for e in es:
+            e.iterate_async(steps)
+        for e in es:
+            e.wait()
+    launches = [e.last_timing()[1] for e in es]
+    assert min(launches[:3]) > 100 and max(launches[3:]) <= 4, launches
+    for e in es:
+        _same(e, ref)
 
 
 @pytest.mark.parametrize("n", [(20, 21, 22), (33, 30, 34), (22, 37, 65)])
@@ -278,3 +302,18 @@ def test_random_scenes_on_the_default_engine(seed):
     for p in op.probes:
         if p.enabled and p.type in (0, 1):
             assert eng.probe_now(p) == ref.probe_now(p)
+
+
+@pytest.mark.parametrize("n,wall", [((12, 11, 32), BC_PEC), ((21, 20, 22), BC_PML), ((91, 92, 90), BC_MUR)])
+def test_engines_that_always_run_resident(n, wall):
+    """Grids so small that the SMs hold several, and large ones with Mur faces."""
+    cop = CompressedOperator(Operator(_scene(n, wall)))
+    es = [Engine(cop, max_timesteps=300, probe_interval=7) for _ in range(3)]
+    ref = Engine(cop, max_timesteps=300, probe_interval=7, kernel="tma")
+    ref.iterate(100)
+    for e in es:
+        e.iterate_async(100)
+    for e in es:
+        e.wait()
+        assert e.last_timing()[1] <= 5
+        _same(e, ref)

@@ -1081,46 +1081,86 @@ static int queue_half_steps(fdtd_engine_t e, uint32_t n) {
     return FDTD_OK;
 }
 
-// n timesteps, run by run: a resident run has the whole GPU, so it is chosen
-// while no other engine of the device has timesteps in flight, and looked at
-// again for each run (two runs are queued ahead).  Engines that share the GPU
-// overlap better on the half-step kernels (us per timestep of all, resident /
-// half-steps: 8 x 41^3 PEC 21.7 / 14.4, 4 x 91^3 38.6 / 29.3, 8 x 47 x 33 x 61
-// UPML 32.5 / 20.2).
-static int queue_steps(fdtd_engine_t e, uint32_t n) {
-    int rc;
-    if (e->resident && n > 0 && !e->res_ready) {
-        if ((rc = setup_resident(e))) return rc;
-        e->resident = e->res_ready;
+// From how many engines in flight on resident runs, one engine after the other,
+// are the faster way; time of a timestep (us) from measurements, resident and
+// as a share of the GPU's throughput on half-steps: 65^3 PEC 4.1 / 4.3, 91^3 9.7
+// / 9.9, 102^3 14.4 / 16.2; UPML 41^3 3.2 / 2.9, 61^3 4.8 / 7.7, 81^3 10.8 /
+// 15.6; dispersive 41 x 46 x 51 4.9 / 4.1, 65 x 71 x 61 9.5 / 12.2; Mur 34^3 3.3
+// / 3.0, 91 x 92 x 90 9.9 / 12.8.  Fewer engines than that have less to move
+// than L2 holds and overlap better (4 x 91^3 PEC 38 us resident, 26 on
+// half-steps).  Always resident: grids so small that an SM holds blocks of
+// several of them (26 x 11 x 32: 2 engines 2.7 us resident, 7.5 on half-steps,
+// 16 engines 13.6, 18.8; 21^3 UPML 2.7, 8.7; 13.6, 21.6), and large ones with
+// Mur faces, whose timesteps are four launches (91 x 92 x 90: 2 engines 20, 31;
+// 16 engines 160, 234; 61^3 11, 24, but 91, 88).
+static int crowd_size(const fdtd_engine_s* e) {
+    const double n = (double)e->N[0] * e->N[1] * e->N[2];
+    if (3 * e->res_threads <= 672 && 2 * (e->res_smem + 1024) <= 227 * 1024) return 1;
+    if (e->mur.nface && n >= 3e5) return 1;
+    double res, half;
+    if (e->mur.nface || e->rlc.count) {
+        res = 2.9 + 9.3e-6 * n;
+        half = 1.9 + 14.5e-6 * n;
+    } else if (e->feat & FEAT_ADE) {
+        res = 2.5 + 25e-6 * n;
+        half = n / 23e3;
+    } else if (e->feat & FEAT_UPML) {
+        res = 2.2 + 16.5e-6 * n;
+        half = n / 32e3;
+    } else {
+        res = 1.9 + 11.3e-6 * n;
+        half = n / 62e3;
     }
-    if (!e->resident) return queue_half_steps(e, n);
+    if (res >= 0.9 * half) return 1 << 30;
+    return e->mur.nface || e->rlc.count || e->feat ? 4 : 6;
+}
+
+// n timesteps, run by run.  A resident run has the whole GPU: an engine alone
+// runs resident, looking again at each run (two are queued ahead) whether it
+// still is alone.  A few engines that share the GPU overlap better on the
+// half-step kernels (us per timestep of all, resident / half-steps: 8 x 41^3
+// PEC 21.7 / 14.4, 4 x 91^3 38.6 / 29.3, 8 x 47 x 33 x 61 UPML 32.5 / 20.2),
+// many only where crowd_size does not say otherwise (16 x 61^3 UPML 77 / 124).
+// An asynchronous call, after which others may follow, counts as alone if the
+// engine's last one was.
+static int queue_runs(fdtd_engine_t e, uint32_t n, bool sync) {
+    const int crowd = crowd_size(e), among = InFlight::count(e->device);
+    auto resident = [&](int c) { return (c == 1 && (sync || e->async_alone)) || c >= crowd; };
+    int rc;
+    e->async_call = !sync;
     uint32_t left = n;
     for (uint32_t k = 0; left > 0; ++k) {
-        if (k >= 2) CK(cudaEventSynchronize(e->ev_run[k & 1]));
-        const uint32_t run = resident_run(e, left);
+        if (sync && k >= 2) CK(cudaEventSynchronize(e->ev_run[k & 1]));
         // A single timestep pays for a whole trip of the state into shared memory
         // and back: without Mur or RLC launches beside the half-steps those are
         // faster (us per call, resident / half-steps: 65^3 PEC 40 / 40, 91^3 49 /
         // 46, 102^3 61 / 52, 65 x 71 x 61 dispersive 49 / 44; with Mur 51 x 42 x 61
         // 41 / 56).  Two timesteps are faster resident on all of these.
-        if (InFlight::count(e->device) == 1 && (left > 1 || e->mur.nface || e->rlc.count)) {
+        bool res = e->resident && resident(sync ? InFlight::count(e->device) : among) &&
+                   (left > 1 || e->mur.nface || e->rlc.count);
+        if (res && !e->res_ready) {
+            if ((rc = setup_resident(e))) return rc;
+            res = e->resident = e->res_ready;
+        }
+        const uint32_t run = e->resident && (sync || res) ? resident_run(e, left) : left;
+        if (res) {
             if ((rc = launch_resident(e, run, e->stream))) return rc;
             e->ts += run;
         } else if ((rc = queue_half_steps(e, run))) {
             return rc;
         }
         left -= run;
-        if (left) CK(cudaEventRecord(e->ev_run[k & 1], e->stream));
+        if (sync && left) CK(cudaEventRecord(e->ev_run[k & 1], e->stream));
     }
     return FDTD_OK;
 }
 
 // An iterate call up to its wait.
-static int queue_call(fdtd_engine_t e, uint32_t n, int (*queue)(fdtd_engine_t, uint32_t)) {
+static int queue_call(fdtd_engine_t e, uint32_t n, bool sync) {
     int rc;
     if ((rc = begin_steps(e, &n))) return rc;
     e->flight.enter(e->device);
-    rc = queue(e, n);
+    rc = queue_runs(e, n, sync);
     if (rc == FDTD_OK) {
         const cudaError_t ce = cudaEventRecord(e->ev1, e->stream);
         if (ce != cudaSuccess) {
@@ -1134,7 +1174,7 @@ static int queue_call(fdtd_engine_t e, uint32_t n, int (*queue)(fdtd_engine_t, u
 }
 
 int fdtd_engine_iterate(fdtd_engine_t e, uint32_t n) {
-    const int rc = queue_call(e, n, queue_steps);
+    const int rc = queue_call(e, n, true);
     return rc ? rc : fdtd_engine_wait(e);
 }
 
@@ -1144,6 +1184,7 @@ int fdtd_engine_wait(fdtd_engine_t e) {
     CK(cudaSetDevice(e->device));
     e->pending = false;
     const cudaError_t ce = cudaEventSynchronize(e->ev1);
+    if (e->async_call) e->async_alone = e->flight.alone();
     e->flight.leave();
     CK(ce);
     float ms = 0;
@@ -1152,9 +1193,9 @@ int fdtd_engine_wait(fdtd_engine_t e) {
     return check_error_word(e);
 }
 
-// Engines stepped this way share the GPU: the half-step kernels.
+// Engines stepped this way are meant to share the GPU.
 int fdtd_engine_iterate_async(fdtd_engine_t e, uint32_t n) {
-    return queue_call(e, n, queue_half_steps);
+    return queue_call(e, n, false);
 }
 
 int fdtd_engine_set_fd(fdtd_engine_t e, const double* freqs, uint32_t nfreq, uint32_t fd_interval) {

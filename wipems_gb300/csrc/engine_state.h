@@ -31,21 +31,30 @@ namespace wipems {
 // How many engines and batches of this process have timesteps in flight on a
 // device; one that has them enters, and leaves when they are done or it ends.
 class InFlight {
-    static std::atomic<int>& at(int device) {
-        static std::atomic<int> n[64];
-        return n[device & 63];
+    struct Device {
+        std::atomic<int> now{0};
+        std::atomic<unsigned> entered{0};
+    };
+    static Device& at(int device) {
+        static Device d[64];
+        return d[device & 63];
     }
     int device = -1;
+    unsigned mine = 0;
+    bool first = false;
 
   public:
-    static int count(int device) { return at(device).load(std::memory_order_relaxed); }
+    static int count(int device) { return at(device).now.load(std::memory_order_relaxed); }
     void enter(int dev) {
         leave();
         device = dev;
-        at(dev).fetch_add(1, std::memory_order_relaxed);
+        first = at(dev).now.fetch_add(1, std::memory_order_relaxed) == 0;
+        mine = at(dev).entered.fetch_add(1, std::memory_order_relaxed) + 1;
     }
+    // whether no other was in flight at any time since enter()
+    bool alone() const { return device >= 0 && first && at(device).entered.load(std::memory_order_relaxed) == mine; }
     void leave() {
-        if (device >= 0) at(device).fetch_sub(1, std::memory_order_relaxed);
+        if (device >= 0) at(device).now.fetch_sub(1, std::memory_order_relaxed);
         device = -1;
     }
     ~InFlight() { leave(); }
@@ -144,6 +153,8 @@ struct fdtd_engine_s {
     bool use_graphs = true;
     bool pending = false;    // an asynchronous iterate was launched, not yet waited for
     InFlight flight;
+    bool async_call = false;    // the call in flight is asynchronous
+    bool async_alone = false;   // the last asynchronous call had the GPU to itself
     double end_crit = 0;     // > 0: stop on the device (energy decay or stop_ts)
     uint32_t stop_ts = 0;
     bool done = false;       // as of the last control-word read
