@@ -25,7 +25,9 @@
 //   102^3 PEC 18.9 -> 15.1              61 x 51 x 71 UPML + RLC 13.8 -> 6.3
 //   51 x 42 x 61 Mur 17.3 -> 4.2        91 x 92 x 90 Mur 25.0 -> 10.1
 //   21 x 4 x 1001 Mur, Drude 16.0 -> 3.9 (five launches per timestep before)
-// so every grid that fits runs resident.
+// so an engine that has the GPU to itself runs every grid that fits resident.
+// The same run takes up to 4 % more or less by where its exchange words lie in
+// memory (engines of one grid differ by that).
 //
 // Arithmetic: as update_node (node.cuh).
 #pragma once

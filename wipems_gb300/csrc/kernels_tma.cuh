@@ -331,8 +331,8 @@ __device__ __forceinline__ bool volt_tile(const DevGrid& g, const TmaMaps& m, co
 // plane of the chunk to the lowest: the x+1 voltages of a node are then its
 // own of the plane before, in registers, as the x-1 currents of the voltage
 // update are.  (Marching upwards read them from the next ring stage: a second
-// wait per plane and one more plane loaded per chunk.)  es/ec/hs/hc: the
-// thread's Kahan sums of V^2 and I^2, accumulated when energy is set.
+// wait per plane and one more plane loaded per chunk.)  With energy set each
+// warp also stores its segment's sums of V^2 and I^2.
 template <typename IdxT, int FEAT, bool GEO, int TY = TMA_TY>
 __device__ __forceinline__ bool curr_tile(const DevGrid& g, const TmaMaps& m, const TileInfo& ti, int bx, int by,
                                           int bz, int XC, int STAGES, float* smem, uint64_t* bars, uint32_t& ring,
@@ -497,9 +497,9 @@ __global__ void __launch_bounds__(TY * 32, MINB) k_curr_tma(const DevGrid g, con
     if (*g.d_done) return;
     init_ring(bars, STAGES);
     uint32_t ring = 0;
-    // x-chunks (and the planes in them) in descending order: blocks are dispatched roughly in
-    // blockIdx order, and the voltage kernel before this one ended on the
-    // highest chunks, whose voltages (just written) and currents (just read)
+    // x-chunks (and the planes in them) in descending order: blocks are
+    // dispatched roughly in blockIdx order, and the voltage kernel before this
+    // one ended on the highest chunks, whose voltages (just written) and currents (just read)
     // are still partly in L2.  The next voltage kernel, in ascending order,
     // starts where this one ends.  No block reads what another block of the
     // same kernel writes, so the order does not change any result.
