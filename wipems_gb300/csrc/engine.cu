@@ -1142,7 +1142,9 @@ static int queue_runs(fdtd_engine_t e, uint32_t n, bool sync) {
             if ((rc = setup_resident(e))) return rc;
             res = e->resident = e->res_ready;
         }
-        const uint32_t run = e->resident && (sync || res) ? resident_run(e, left) : left;
+        uint32_t run = e->resident && (sync || res) ? resident_run(e, left) : left;
+        if (!res && e->interval && (e->ts + run) % e->interval)  // to the end of an interval: its graph
+            run = std::min(left, run + e->interval - (e->ts + run) % e->interval);
         if (res) {
             if ((rc = launch_resident(e, run, e->stream))) return rc;
             e->ts += run;
